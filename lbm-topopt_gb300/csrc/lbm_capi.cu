@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/lbmgpu.h"
+#include "fixed_model.hpp"
 #include "lbm_device.cuh"
 #include "lbm_ops.h"
 #include "state_pool.hpp"
@@ -165,6 +166,11 @@ struct lbm_handle {
   void* gamma = nullptr;
   void* lam[2] = {nullptr, nullptr};
   int lcur = 0;
+  FixedModel fix = {};                 // fixed-point form of the FP64 collision
+  unsigned long long* im = nullptr;    // its porosity planes (KParams::im, dimult)
+  double* dimult = nullptr;
+  unsigned long long* om6 = nullptr;   // and the thermal lattice's (om6, domega)
+  double* domega = nullptr;
   double* sens = nullptr;
   double* partial = nullptr;
   unsigned* counter = nullptr;
@@ -393,7 +399,8 @@ void destroy_buffers(lbm_handle* h) {
   for (void* s : h->slots)
     if (s) cudaFree(s);
   h->slots.clear();
-  void* ps[] = {h->gamma, h->sens, h->partial, h->counter, h->jdev, h->stage, h->init_mac};
+  void* ps[] = {h->gamma,  h->im,      h->dimult,  h->om6,  h->domega, h->sens,
+                h->partial, h->counter, h->jdev, h->stage, h->init_mac};
   for (void* p : ps)
     if (p) cudaFree(p);
   for (int k = 0; k < LBM_MAX_BC; ++k) {
@@ -403,6 +410,9 @@ void destroy_buffers(lbm_handle* h) {
     h->bcprof_f[k] = nullptr;
   }
   h->gamma = h->sens = h->partial = nullptr;
+  h->im = nullptr;
+  h->dimult = h->domega = nullptr;
+  h->om6 = nullptr;
   h->counter = nullptr;
   h->jdev = h->stage = h->init_mac = nullptr;
   for (cudaEvent_t& e : h->ev)
@@ -495,6 +505,11 @@ KParams base_params(const lbm_handle* h, int t) {
   p.gamma = h->gamma;
   p.sens = h->sens;
   p.sens_atomic = h->sens_atomic ? 1 : 0;
+  p.fix = h->fix;
+  p.im = h->im;
+  p.dimult = h->dimult;
+  p.om6 = h->om6;
+  p.domega = h->domega;
   return p;
 }
 
@@ -804,6 +819,15 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   ALLOC(h->lam[0], adjoint_bytes(h));
   ALLOC(h->lam[1], adjoint_bytes(h));
   ALLOC(h->gamma, (size_t)h->P * h->gam_bytes);
+  h->fix = fixed_model(c);
+  if (h->fix.ok) {
+    ALLOC(h->im, (size_t)h->P * sizeof(unsigned long long));
+    ALLOC(h->dimult, (size_t)h->P * sizeof(double));
+    if (c.lattice == LBM_D2Q9_D2Q5) {
+      ALLOC(h->om6, (size_t)h->P * sizeof(unsigned long long));
+      ALLOC(h->domega, (size_t)h->P * sizeof(double));
+    }
+  }
   ALLOC(h->sens, (size_t)h->P * sizeof(double));
   ALLOC(h->partial, h->partial_cap * sizeof(double));
   ALLOC(h->counter, sizeof(unsigned));

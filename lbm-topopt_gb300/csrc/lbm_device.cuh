@@ -249,6 +249,18 @@ struct ModelParams {
   C obj_p[2];                  // objective parameters (regenerator efficiency: Ti, w/D)
 };
 
+// Constants of a model's collision in 64-bit fixed point (lbm_fixed.cuh says
+// what c[] holds for each operator), filled once per handle by the host.
+struct FixedModel {
+  int ok;                            // the model has a fixed-point form with these constants
+  int rest;                          // cells at rest take the FP64 operators
+  int we3;                           // the D3Q19 MRT weight we differs from 3
+  int wej_neg, wxx_neg, we3_neg;     // signs of the three below: 0 or -1
+  unsigned long long c[12];          // factors below 1, times 2^64
+  unsigned long long wej, wxx, we3c; // |wej/4|, |wxx| and |(we - 3)/4| times 2^62
+  unsigned long long cv;             // the dissipation's viscous factor (9/2) nu omega^2 times 2^64
+};
+
 struct KParams {
   int nx, ny, nz;
   long long P;       // plane stride in elements
@@ -283,6 +295,12 @@ struct KParams {
   void* lam_out;           // eta_t
   double* sens;
   int sens_atomic;         // add to dJ/dgamma with an atomic (reverse steps that fit in L2)
+  // FP64 storage: the collisions in fixed point
+  FixedModel fix;
+  const unsigned long long* im;   // imult * 2^64 of the design, all ones where it does not fit
+  const double* dimult;           // d(imult)/d(gamma) of the design
+  const unsigned long long* om6;  // thermal lattice: om_T / 6 * 2^64, all ones where it does not fit
+  const double* domega;           // thermal lattice: d(om_T)/d(gamma)
 };
 
 template <class C>

@@ -16,6 +16,7 @@
 #pragma once
 
 #include "lbm_device.cuh"
+#include "lbm_fixed.cuh"
 #include "lbm_ops.h"
 
 namespace lbm {
@@ -44,7 +45,8 @@ struct Occupancy {
 };
 template <int LAT, int COLL>
 struct Occupancy<LAT, COLL, double> {
-  static constexpr int fwd = 1, adj = 1, adj_lean = 1, adj_lean_batch = 1;
+  static constexpr int fwd = LAT == LAT_D2Q9 ? 3 : 2, adj = LAT == LAT_D2Q9 ? 2 : 1;
+  static constexpr int adj_lean = adj, adj_lean_batch = adj;
   static constexpr bool has_lean = false;
 };
 
@@ -263,6 +265,115 @@ __device__ __forceinline__ typename Store<S>::C forward_cell_from(const KParams&
   return objv;
 }
 
+// FP64 operators of the cells that the fixed-point ones do not take: out of
+// line, so that they cost the others neither registers nor instruction cache.
+template <int LAT, int COLL>
+__device__ __noinline__ void collide_fp64(double* f, double g, const KParams& p) {
+  const double imult = 0.5 * (p.md.pbb_scale * bp(g, p.md.pbb_q));
+  double rho, jx, jy, jz, T;
+  flow_collide<LAT, COLL>(f, imult, rho, jx, jy, jz, p);
+  if constexpr (LAT == LAT_D2Q9_D2Q5) thermal_collide(f + 9, jx, jy, g, T, p);
+}
+
+template <int LAT, int COLL>
+__device__ __noinline__ void reverse_fp64(const double* f, double* lam, double g, double& dg,
+                                          const KParams& p) {
+  const double imult = 0.5 * (p.md.pbb_scale * bp(g, p.md.pbb_q));
+  const double dimult = 0.5 * (p.md.pbb_scale * bp_diff(g, p.md.pbb_q));
+  double uxR = 0., uyR = 0.;
+  if constexpr (LAT == LAT_D2Q9_D2Q5) {
+    double rho, jx, jy, jz;
+    flow_macros<LAT>(f, rho, jx, jy, jz);
+    thermal_reverse(f + 9, lam + 9, jx, jy, g, uxR, uyR, dg, p);
+  }
+  flow_reverse<LAT, COLL>(f, lam, imult, dimult, dg, p);
+  if constexpr (LAT == LAT_D2Q9_D2Q5) {
+    static_for<9>([&](auto I) {
+      constexpr int i = decltype(I)::value;
+      lam[i] += e_dot<LAT, i>(uxR, uyR, 0.);
+    });
+  }
+}
+
+// Whether the collision runs in fixed point: FP64 storage.
+template <class S>
+constexpr bool kFixed = std::is_same<S, double>::value;
+
+// the porosity plane's value where the fixed-point form takes it (0 .. 2^63)
+__device__ __forceinline__ bool fixed_porosity(unsigned long long im) {
+  return (unsigned)(im >> 32) <= 0x80000000u;
+}
+
+// What the design contributes to a cell of a fixed-point step (KParams).
+template <int LAT>
+struct FixedDesign {
+  unsigned long long im, om6 = 0ull;
+  __device__ __forceinline__ FixedDesign(const KParams& p, int c) : im(p.im[c]) {
+    if constexpr (LAT == LAT_D2Q9_D2Q5) om6 = p.om6[c];
+  }
+  __device__ __forceinline__ bool ok() const { return fixed_porosity(im) && om6 != ~0ull; }
+};
+
+// forward_cell_from for FP64 storage with the collision in fixed point
+// (lbm_fixed.cuh).
+template <int LAT, int COLL, bool WARP>
+__device__ __forceinline__ double forward_cell_fixed(const KParams& p, int x, int y, int z, int c,
+                                                     double* f, const FixedDesign<LAT>& des,
+                                                     bool in) {
+  using L = Lattice<LAT>;
+  constexpr bool THERMAL = LAT == LAT_D2Q9_D2Q5;
+  const double* __restrict__ gamma = (const double*)p.gamma;
+  double objv = 0.;
+  if (on_bc_face<LAT>(x, y, p)) apply_bcs<LAT, false>(f, x, y, z, p);
+  const bool diss = L::DIM == 2 && p.eval_obj && p.objective == LBM_OBJ_DISSIPATION;
+  if (p.eval_obj && !diss) objv = objective_cell<LAT, false>(f, gamma[c], x, y, z, p);
+  fx::Window w;
+  fx::i64 xi[L::QF];
+  static_for<L::QF>([&](auto Q_) {
+    constexpr int q = decltype(Q_)::value;
+    xi[q] = w.template load<LAT, q>(f[q]);
+  });
+  bool ok = w.template ok<LAT>(xi) && des.ok();
+  if (p.fix.rest) ok = ok && !fx::at_rest<LAT>(xi);
+  fx::Block bt;
+  if constexpr (THERMAL) {
+    bt.template measure<5, fx::kThermalBits>(f + 9);
+    ok = ok && (bt.zero || bt.ok);
+  }
+  if (ok) {
+    if constexpr (L::DIM == 2) {
+      if (diss) objv = fx::dissipation2(xi, des.im, p.md.obj_weight, p.md.cv_diss);
+    }
+    if constexpr (THERMAL) {
+      double T = 0.;
+      if (!bt.zero) {
+        const fx::Pairs2 u(xi);
+        const fx::Thermal t(f + 9, bt, u.jx, u.jy);
+        T = fx::to_double(t.T, bt.k);
+        fx::thermal_collide(t, bt, des.om6, f + 9);
+      }
+      if (p.md.heat_rate != 0.) {
+        const double hs = (1. - gamma[c]) * p.md.heat_rate * (p.md.heat_T - T);
+        static_for<5>([&](auto I) {
+          constexpr int i = decltype(I)::value + 9;
+          f[i] += L::w(i) * hs;
+        });
+      }
+    }
+    fx::collide<LAT, COLL>(xi, fx::Factor(des.im), p.fix, f);
+  } else {
+    if constexpr (L::DIM == 2) {
+      if (diss) objv = ObjDissipation::evaluate<LAT, false>(f, gamma[c], x, y, z, p);
+    }
+    double t[L::Q];
+    static_for<L::Q>([&](auto Q_) { t[decltype(Q_)::value] = f[decltype(Q_)::value]; });
+    collide_fp64<LAT, COLL>(t, gamma[c], p);
+    static_for<L::Q>([&](auto Q_) { f[decltype(Q_)::value] = t[decltype(Q_)::value]; });
+  }
+  push_all<LAT, double>(f, (double*)p.fout, c, x, y, z, take_interior<LAT, WARP>(in, x, y, z, p), p);
+  return objv;
+}
+
 // Forward step of cell (x,y,z); returns its objective contribution F(f_t).
 // in: warp_interior of the calling warp, read with WARP.
 template <int LAT, int COLL, class S, bool WARP>
@@ -276,6 +387,10 @@ __device__ __forceinline__ typename Store<S>::C forward_cell(const KParams& p, i
     const int c = (z * p.ny + y) * p.nx + x;
     C f[L::Q];
     load_state<LAT, S>(f, (const S*)p.fin, c, (int)p.P);
+    if constexpr (kFixed<S>) {
+      if (p.fix.ok)
+        return forward_cell_fixed<LAT, COLL, WARP>(p, x, y, z, c, f, FixedDesign<LAT>(p, c), in);
+    }
     objv = forward_cell_from<LAT, COLL, S, WARP>(p, x, y, z, c, f, C(((const G*)p.gamma)[c]), in);
   }
   return objv;
@@ -297,6 +412,109 @@ __device__ __forceinline__ void add_sensitivity(double* sens, int c, double dg, 
     sens[c] += dg;
 }
 
+// The temperature lattice of a reverse step: lam[9..13] through the transposed
+// collision, its share of the flow's adjoint into lam[0..8]; returns its share
+// of dJ/dgamma.  g, l: scales of the cell's temperatures and of their adjoint.
+__device__ __forceinline__ double thermal_reverse_cell(const KParams& p, int c, const double* f,
+                                                       double* lam, const fx::Pairs2& u,
+                                                       const fx::Block& g, const fx::Block& l,
+                                                       unsigned long long om6) {
+  double dg = 0., T = 0.;
+  if (!g.zero) {
+    const fx::Thermal t(f + 9, g, u.jx, u.jy);
+    T = fx::to_double(t.T, g.k);
+    // sum (g_eq - g) lam, the derivative by om_T
+    double r = 2. * (fx::to_double(t.excess<0>(), g.k) * lam[9]);
+    static_for<4>([&](auto I) {
+      constexpr int i = decltype(I)::value + 1;
+      r += fx::to_double(t.excess<i>(), g.k) * lam[9 + i];
+    });
+    dg = r * (1. / 6.) * p.domega[c];
+  }
+  const fx::ThermalAdjoint a = fx::thermal_reverse(lam + 9, l, u.jx, u.jy, om6);
+  // 3 T om/6 (lam_4 - lam_2), and alike in y
+  const double tom = T * (3. * fx::to_double((fx::i64)(om6 >> 1), 63));
+  const double uxR = tom * a.dx, uyR = tom * a.dy;
+  static_for<9>([&](auto I) {
+    constexpr int i = decltype(I)::value;
+    if constexpr (i != 0) lam[i] += e_dot<LAT_D2Q9, i>(uxR, uyR, 0.);
+  });
+  if (p.md.heat_rate != 0.) {
+    const double hsR = a.sum6 * (1. / 6.), hr = p.md.heat_rate;
+    const double heat = -(1. - ((const double*)p.gamma)[c]) * hr * hsR;
+    static_for<5>([&](auto I) { lam[9 + decltype(I)::value] += heat; });
+    dg += -hr * (p.md.heat_T - T) * hsR;
+  }
+  return dg;
+}
+
+// Reverse step of cell c for FP64 storage with the transposed collision in
+// fixed point.
+template <int LAT, int COLL, bool WARP>
+__device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int y, int z, int c,
+                                                   bool in) {
+  using L = Lattice<LAT>;
+  constexpr bool THERMAL = LAT == LAT_D2Q9_D2Q5;
+  double lam[L::Q], f[L::Q];
+  pull_all<LAT, double, double>(lam, (const double*)p.lam_in, c, x, y, z,
+                                take_interior<LAT, WARP>(in, x, y, z, p), p);
+  load_state<LAT, double>(f, (const double*)p.fin, c, (int)p.P);
+  const FixedDesign<LAT> des(p, c);
+  const double dimult = p.dimult[c];
+  if (on_bc_face<LAT>(x, y, p)) apply_bcs<LAT, false>(f, x, y, z, p);
+  double dg = 0.;
+  fx::Block b, l, g;
+  b.template measure<L::QF>(lam);
+  bool zero = b.zero, ok = b.zero || b.ok;
+  if constexpr (THERMAL) {
+    l.template measure<5, fx::kThermalBits>(lam + 9);
+    g.template measure<5, fx::kThermalBits>(f + 9);
+    zero = zero && l.zero;
+    ok = ok && (l.zero || l.ok) && (g.zero || g.ok);
+  }
+  const bool diss = L::DIM == 2 && p.eval_obj && p.objective == LBM_OBJ_DISSIPATION;
+  // cells that no adjoint has reached yet keep their zeros
+  if (!zero || diss) {
+    fx::Window w;
+    fx::i64 xi[L::QF];
+    static_for<L::QF>([&](auto Q_) {
+      constexpr int q = decltype(Q_)::value;
+      xi[q] = w.template load<LAT, q>(f[q]);
+    });
+    ok = ok && w.template ok<LAT>(xi) && des.ok();
+    if (p.fix.rest) ok = ok && !fx::at_rest<LAT>(xi);
+    if (ok) {
+      if (!b.zero) dg = dimult * fx::reverse<LAT, COLL>(xi, lam, b, fx::Factor(des.im), p.fix);
+      if constexpr (THERMAL) {
+        if (!l.zero) dg += thermal_reverse_cell(p, c, f, lam, fx::Pairs2(xi), g, l, des.om6);
+      }
+      if constexpr (L::DIM == 2) {
+        if (diss)
+          dg += dimult * fx::dissipation2_source(xi, des.im, p.md.obj_weight, p.fix.cv, lam);
+      }
+    } else {
+      double t[L::Q], u[L::Q], d = 0.;
+      static_for<L::Q>([&](auto Q_) {
+        constexpr int q = decltype(Q_)::value;
+        t[q] = f[q];
+        u[q] = lam[q];
+      });
+      reverse_fp64<LAT, COLL>(t, u, ((const double*)p.gamma)[c], d, p);
+      dg = d;
+      static_for<L::Q>([&](auto Q_) { lam[decltype(Q_)::value] = u[decltype(Q_)::value]; });
+    }
+  }
+  if (p.eval_obj && !(diss && ok))
+    objective_source<LAT, false>(f, ((const double*)p.gamma)[c], lam, dg, x, y, z, p);
+  if (on_bc_face<LAT>(x, y, p)) adjoint_bcs<LAT>(lam, x, y, z, p);
+  double* __restrict__ lout = (double*)p.lam_out;
+  static_for<L::Q>([&](auto Q_) {
+    constexpr int q = decltype(Q_)::value;
+    lout[q * (int)p.P + c] = lam[q];
+  });
+  add_sensitivity<LAT>(p.sens, c, dg, p.sens_atomic);
+}
+
 // Reverse step of cell (x,y,z); in: warp_interior of the calling warp, read
 // with WARP.
 template <int LAT, int COLL, class S, bool WARP>
@@ -308,6 +526,12 @@ __device__ __forceinline__ void adjoint_cell(const KParams& p, int x, int y, int
   constexpr bool SHIFT = Store<S>::SHIFT;
   if (x >= p.nx || y >= p.ny) return;
   const int c = (z * p.ny + y) * p.nx + x;
+  if constexpr (kFixed<S>) {
+    if (p.fix.ok) {
+      adjoint_cell_fixed<LAT, COLL, WARP>(p, x, y, z, c, in);
+      return;
+    }
+  }
   const A* __restrict__ lin = (const A*)p.lam_in;
   A* __restrict__ lout = (A*)p.lam_out;
   C lam[L::Q];
@@ -679,6 +903,30 @@ __global__ void k_gamma(const double* __restrict__ src, G* __restrict__ dst, lon
   if (i < n) dst[i] = G(src[i]);
 }
 
+// FP64 storage: the design and what the fixed-point collisions read instead
+// of evaluating it at every step: imult * 2^64 (imult in [0, 1/2]; all ones
+// elsewhere, which sends the cell to the FP64 operators), d(imult)/d(gamma) and,
+// on the thermal lattice, om_T / 6 * 2^64 (om_T in (0, 2], or all ones) and
+// d(om_T)/d(gamma).
+static __global__ void k_gamma_fixed(const double* __restrict__ src, KParams p, long long n) {
+  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double g = src[i];
+  ((double*)p.gamma)[i] = g;
+  const double imult = 0.5 * (p.md.pbb_scale * bp(g, p.md.pbb_q));
+  const_cast<unsigned long long*>(p.im)[i] =
+      imult >= 0. && imult <= 0.5 ? __double2ull_rn(imult * 18446744073709551616.) : ~0ull;
+  const_cast<double*>(p.dimult)[i] = 0.5 * (p.md.pbb_scale * bp_diff(g, p.md.pbb_q));
+  if (p.om6) {
+    const double r = ramp(g, p.md.ramp_q, p.md.ramp_ck), den = 3. * p.md.diff * r + 0.5;
+    const double om = 1. / den;
+    const_cast<unsigned long long*>(p.om6)[i] =
+        om > 0. && om <= 2. ? __double2ull_rn(om * 3074457345618258602.7) : ~0ull;   // 2^64 / 6
+    const_cast<double*>(p.domega)[i] =
+        (-1. / (den * den)) * 3. * p.md.diff * ramp_diff(g, p.md.ramp_q, p.md.ramp_ck);
+  }
+}
+
 // ---------------------------------------------------------------------------
 
 // Launch of a kernel that begins with step_prologue, with programmatic stream
@@ -770,6 +1018,10 @@ struct OpsImpl {
         break;
       case K_GAMMA: {
         long long n = (long long)p.nx * p.ny * p.nz;
+        if (p.im) {
+          k_gamma_fixed<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(aux, p, n);
+          break;
+        }
         k_gamma<typename GammaT<S>::T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
             aux, (typename GammaT<S>::T*)p.gamma, n);
         break;

@@ -1,0 +1,83 @@
+"""FP64 storage on the GPU, whose collisions run in fixed point where a cell's
+populations allow it (lbm_fixed.cuh), against the oracle on lattices whose
+cells lie inside, outside and across the accepted range (velocities and
+densities to both sides of its limits), and with designs that the porosity
+plane does not hold.  Tolerance 1e-12 as for every FP64 comparison."""
+import numpy as np
+import pytest
+
+import lbmgpu as G
+import workloads as W
+from helpers import rel_inf
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def config(name):
+    if name == "d3q19_mrt":
+        return W.duct_3d(13, 9, 7, nsteps=12), W.design_3d(13, 9, 7, 3)
+    if name == "d2q9_bgk":
+        return W.channel_2d(21, 14, nsteps=12, amp=0.2, period=9.0), W.design_2d(21, 14, 3)
+    if name == "d2q9_mrt":
+        return W.channel_2d(33, 9, nsteps=12, collision=G.MRT), W.design_2d(33, 9, 4)
+    if name == "d2q9_bgk_dissipation":
+        return (W.channel_2d(40, 23, nsteps=12, objective=G.OBJ_DISSIPATION, amp=0.2, period=9.0),
+                W.design_2d(40, 23, 5))
+    if name == "d3q19_bgk":
+        return W.duct_3d(9, 11, 6, nsteps=12).replace(collision=G.BGK), W.design_3d(9, 11, 6, 6)
+    if name == "thermal":
+        return W.thermal_2d(35, 18, nsteps=12, period=9.0), W.thermal_design(35, 18, 7)
+    if name == "regenerator":
+        return (W.regenerator_2d(30, 17, n_unsteady=12, objective=G.OBJ_DOMAIN_TEMPERATURE),
+                W.regenerator_design(30, 17, 8))
+    raise KeyError(name)
+
+
+def macros(cfg, drho, u, seed):
+    rng = np.random.default_rng(seed)
+    m = np.zeros((cfg.ncells, cfg.nmac))
+    m[:, 0] = 1 + drho * rng.uniform(-1, 1, cfg.ncells)
+    dim = 3 if cfg.lattice == G.D3Q19 else 2
+    m[:, 1:1 + dim] = u * rng.uniform(-1, 1, (cfg.ncells, dim))
+    if cfg.lattice == G.D2Q9_D2Q5:
+        m[:, 3] = rng.uniform(0, 1, cfg.ncells)
+    return m.ravel()
+
+
+MODELS = ["d3q19_mrt", "d2q9_bgk", "d2q9_mrt", "d2q9_bgk_dissipation", "d3q19_bgk", "thermal",
+          "regenerator"]
+
+
+@pytest.mark.parametrize("drho,u", [(0.0, 0.02), (0.15, 0.1), (0.6, 0.3)])
+@pytest.mark.parametrize("name", MODELS)
+def test_inside_across_and_outside_the_range(orc, name, drho, u):
+    cfg, gamma = config(name)
+    mac = macros(cfg, drho, u, 5)
+    with G.Handle(cfg) as h:
+        h.set_design(gamma)
+        h.init_equilibrium(mac)
+        J, js = h.forward(12, per_step=True)
+        f = h.populations()
+        Jg, s, _ = h.gradient(12, 3)
+    fo, jo, _ = orc.forward(cfg, gamma, 12, macros=mac)
+    assert rel_inf(f, fo) < TOL
+    assert rel_inf(js, jo) < TOL
+    Jo, so = orc.gradient(cfg, gamma, 12, macros=mac)
+    assert abs(Jg - Jo) <= TOL * abs(jo).max() * 12
+    assert rel_inf(s, so) < TOL
+
+
+@pytest.mark.parametrize("name", MODELS)
+def test_large_drag_leaves_the_porosity_plane(orc, name):
+    """interp_scale = 1.6: imult up to 0.8, outside the plane's [0, 1/2]."""
+    cfg, gamma = config(name)
+    cfg = cfg.replace(interp_scale=1.6)
+    with G.Handle(cfg) as h:
+        h.set_design(gamma)
+        h.init_equilibrium()
+        h.forward(12)
+        f = h.populations()
+    fo, _, _ = orc.forward(cfg, gamma, 12)
+    assert rel_inf(f, fo) < TOL
