@@ -45,7 +45,7 @@ struct Occupancy {
 };
 template <int LAT, int COLL>
 struct Occupancy<LAT, COLL, double> {
-  static constexpr int fwd = LAT == LAT_D2Q9 ? 3 : 2, adj = LAT == LAT_D2Q9 ? 2 : 1;
+  static constexpr int fwd = LAT == LAT_D2Q9 ? 3 : 2, adj = 2;
   static constexpr int adj_lean = adj, adj_lean_batch = adj;
   static constexpr bool has_lean = false;
 };
