@@ -29,6 +29,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/lbmgpu.h"
@@ -40,6 +41,8 @@ constexpr int kThreads = 256;
 constexpr int kMaxM = LBM_MAX_REALISATIONS + 1;                 // MMA constraints
 constexpr int kMaxVals = kMaxM + kMaxM * (kMaxM + 1) / 2;      // dual gradient + upper Hessian
 constexpr int kMaxBlocks = 1024;
+// blocks of the reducing kernels: two per SM, so that few block sums remain
+constexpr int kReduceBlocks = 304;
 
 struct Grid {
   int nx, ny, nz;
@@ -49,9 +52,12 @@ struct Grid {
 // One filter stage as the kernels see it.
 struct StageDev {
   int project, ntaps;
+  int reach, reach_z;       // largest |dx|, |dy| and |dz| of a tap
   int box[6];
   double beta, eta, pden;   // pden = tanh(beta eta) + tanh(beta (1 - eta))
+  double pnum;              // tanh(beta eta)
   const int* tap;           // ntaps x (dx, dy, dz), dz then dy then dx ascending
+  const long long* off;     // their index offsets
   const double* w;          // weights R - |d| > 0
   const double* den;        // row sums of the filter matrix (1 outside the box)
 };
@@ -115,38 +121,72 @@ __global__ void k_gather_box(Grid g, const int* __restrict__ b, long long n,
   }
 }
 
-__global__ void k_stage_forward(Grid g, StageDev s, const double* __restrict__ in,
-                                double* __restrict__ keep, double* __restrict__ out) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.n;
-       c += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    cell_xyz(g, c, x, y, z);
+// Cells of the filter kernels: 64 x 4 threads over x and the rows (y, z).
+constexpr int kFilterX = 64, kFilterY = 4;
+__device__ __forceinline__ int rows(const Grid& g) { return g.ny * g.nz; }
+
+// Whether every tap of cell (x,y,z) stays within [lo, hi] of each axis.
+__device__ __forceinline__ bool taps_inside(const StageDev& s, int x, int y, int z, int x0, int x1,
+                                            int y0, int y1, int z0, int z1) {
+  return x - s.reach >= x0 && x + s.reach <= x1 && y - s.reach >= y0 && y + s.reach <= y1 &&
+         z - s.reach_z >= z0 && z + s.reach_z <= z1;
+}
+
+// acc + sum_k w_k v[offset_k], in tap order.  One FP64 multiply-add a tap bounds
+// the filters (two per clock and SM); with the bounds tests and three index
+// loads a tap that they ran with for every cell, the two stages (radii 8 and
+// 4) of a 1024x512 field took 350 us, against 210 us of multiply-adds.
+__device__ __forceinline__ double sum_taps(const StageDev& s, const double* __restrict__ v,
+                                           double acc) {
+  const long long* __restrict__ off = s.off;
+  const double* __restrict__ w = s.w;
+#pragma unroll 4
+  for (int k = 0; k < s.ntaps; ++k) acc += w[k] * v[off[k]];
+  return acc;
+}
+
+__global__ void __launch_bounds__(kThreads) k_stage_forward(Grid g, StageDev s,
+                                                            const double* __restrict__ in,
+                                                            double* __restrict__ keep,
+                                                            double* __restrict__ out) {
+  const int x = blockIdx.x * kFilterX + threadIdx.x;
+  if (x >= g.nx) return;
+  for (int r = blockIdx.y * kFilterY + threadIdx.y; r < rows(g); r += gridDim.y * kFilterY) {
+    const int y = r % g.ny, z = r / g.ny;
+    const long long c = ((long long)z * g.ny + y) * g.nx + x;
     const bool ib = in_box(s.box, x, y, z);
     double v;
     if (!ib) {
       v = in[c];
     } else {
       double acc = 0.;
-      for (int k = 0; k < s.ntaps; ++k) {
-        const int xx = x + s.tap[3 * k], yy = y + s.tap[3 * k + 1], zz = z + s.tap[3 * k + 2];
-        if (xx < 0 || yy < 0 || zz < 0 || xx >= g.nx || yy >= g.ny || zz >= g.nz) continue;
-        acc += s.w[k] * in[((long long)zz * g.ny + yy) * g.nx + xx];
+      if (taps_inside(s, x, y, z, 0, g.nx - 1, 0, g.ny - 1, 0, g.nz - 1)) {
+        acc = sum_taps(s, in + c, acc);
+      } else {
+        for (int k = 0; k < s.ntaps; ++k) {
+          const int xx = x + s.tap[3 * k], yy = y + s.tap[3 * k + 1], zz = z + s.tap[3 * k + 2];
+          if (xx < 0 || yy < 0 || zz < 0 || xx >= g.nx || yy >= g.ny || zz >= g.nz) continue;
+          acc += s.w[k] * in[((long long)zz * g.ny + yy) * g.nx + xx];
+        }
       }
       v = acc / s.den[c];
     }
     keep[c] = v;
-    if (s.project && ib) v = (tanh(s.beta * s.eta) + tanh(s.beta * (v - s.eta))) / s.pden;
+    if (s.project && ib) v = (s.pnum + tanh(s.beta * (v - s.eta))) / s.pden;
     out[c] = v;
   }
 }
 
 // t = (projection derivative at keep) * s / rowsum
-__global__ void k_stage_scale(Grid g, StageDev s, const double* __restrict__ keep,
-                              const double* __restrict__ sin, double* __restrict__ t) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.n;
-       c += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    cell_xyz(g, c, x, y, z);
+__global__ void __launch_bounds__(kThreads) k_stage_scale(Grid g, StageDev s,
+                                                          const double* __restrict__ keep,
+                                                          const double* __restrict__ sin,
+                                                          double* __restrict__ t) {
+  const int x = blockIdx.x * kFilterX + threadIdx.x;
+  if (x >= g.nx) return;
+  for (int r = blockIdx.y * kFilterY + threadIdx.y; r < rows(g); r += gridDim.y * kFilterY) {
+    const int y = r % g.ny, z = r / g.ny;
+    const long long c = ((long long)z * g.ny + y) * g.nx + x;
     double v = sin[c];
     if (s.project && in_box(s.box, x, y, z)) {
       const double th = tanh(s.beta * (keep[c] - s.eta));
@@ -157,18 +197,25 @@ __global__ void k_stage_scale(Grid g, StageDev s, const double* __restrict__ kee
 }
 
 // sout = H^T t: column c gathers the filter rows that hold it (the cone is symmetric)
-__global__ void k_stage_transpose(Grid g, StageDev s, const double* __restrict__ t,
-                                  double* __restrict__ sout) {
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.n;
-       c += (long long)gridDim.x * blockDim.x) {
-    int x, y, z;
-    cell_xyz(g, c, x, y, z);
-    double acc = in_box(s.box, x, y, z) ? 0. : t[c];
-    for (int k = 0; k < s.ntaps; ++k) {
-      const int xx = x + s.tap[3 * k], yy = y + s.tap[3 * k + 1], zz = z + s.tap[3 * k + 2];
-      if (xx < 0 || yy < 0 || zz < 0 || xx >= g.nx || yy >= g.ny || zz >= g.nz) continue;
-      if (!in_box(s.box, xx, yy, zz)) continue;
-      acc += s.w[k] * t[((long long)zz * g.ny + yy) * g.nx + xx];
+__global__ void __launch_bounds__(kThreads) k_stage_transpose(Grid g, StageDev s,
+                                                              const double* __restrict__ t,
+                                                              double* __restrict__ sout) {
+  const int x = blockIdx.x * kFilterX + threadIdx.x;
+  if (x >= g.nx) return;
+  const int* b = s.box;
+  for (int r = blockIdx.y * kFilterY + threadIdx.y; r < rows(g); r += gridDim.y * kFilterY) {
+    const int y = r % g.ny, z = r / g.ny;
+    const long long c = ((long long)z * g.ny + y) * g.nx + x;
+    double acc = in_box(b, x, y, z) ? 0. : t[c];
+    if (taps_inside(s, x, y, z, b[0], b[1], b[2], b[3], b[4], b[5])) {
+      acc = sum_taps(s, t + c, acc);
+    } else {
+      for (int k = 0; k < s.ntaps; ++k) {
+        const int xx = x + s.tap[3 * k], yy = y + s.tap[3 * k + 1], zz = z + s.tap[3 * k + 2];
+        if (xx < 0 || yy < 0 || zz < 0 || xx >= g.nx || yy >= g.ny || zz >= g.nz) continue;
+        if (!in_box(b, xx, yy, zz)) continue;
+        acc += s.w[k] * t[((long long)zz * g.ny + yy) * g.nx + xx];
+      }
     }
     sout[c] = acc;
   }
@@ -182,8 +229,11 @@ __global__ void k_fill(double* v, long long n, double a) {
 
 // ---------------------------------------------------------------------------
 // Fixed-order reductions: every thread accumulates its own elements in index
-// order, warps and blocks combine in a fixed order, a last single-block pass
-// adds the block partials in order.  Results do not depend on timing.
+// order, a block adds its threads' sums in a fixed order, and the last block
+// to finish adds the blocks' sums in a fixed order into host memory.  Results
+// do not depend on timing.  (The blocks' sums used to be added one after the
+// other by one thread per value of a second kernel, 1024 dependent loads: 60%
+// of an MMA step.)
 
 __device__ __forceinline__ double warp_sum_d(double v) {
 #pragma unroll
@@ -196,47 +246,79 @@ __device__ __forceinline__ double warp_max_d(double v) {
   return v;
 }
 
-// part[blockIdx.x * nv + k] = block sum of v[k] (max when use_max)
-__device__ void block_store(double* v, int nv, double* part, bool use_max) {
-  __shared__ double sh[kThreads / 32][kMaxVals];
+struct Reduction {
+  double* part;        // nv x gridDim.x block sums
+  unsigned* counter;   // blocks done, left at zero
+  double* out;         // nv results (mapped host memory)
+};
+
+// out[k] = sum (or max) over the grid of v[k], k < NV; the whole grid calls it
+// once.  Threads first meet in shared memory, a quarter of the FP64 additions
+// of a shuffle tree per warp.
+template <int NV, bool MAX>
+__device__ __forceinline__ void grid_reduce_values(const double* v, const Reduction& r) {
+  constexpr int kAtOnce = 8;   // values per pass: 16 KB of shared memory
+  __shared__ double sh[kAtOnce][kThreads];
+  __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int k = 0; k < nv; ++k) {
-    const double r = use_max ? warp_max_d(v[k]) : warp_sum_d(v[k]);
-    if (lane == 0) sh[wid][k] = r;
+  auto add = [](double a, double b) { return MAX ? fmax(a, b) : a + b; };
+  auto tree = [](double a) { return MAX ? warp_max_d(a) : warp_sum_d(a); };
+#pragma unroll
+  for (int k0 = 0; k0 < NV; k0 += kAtOnce) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kAtOnce; ++k)
+      if (k0 + k < NV) sh[k][threadIdx.x] = v[k0 + k];
+    __syncthreads();
+    if (k0 + wid < NV) {
+      double a = sh[wid][lane];
+#pragma unroll
+      for (int w = 1; w < kThreads / 32; ++w) a = add(a, sh[wid][lane + 32 * w]);
+      a = tree(a);
+      if (lane == 0) r.part[(size_t)(k0 + wid) * gridDim.x + blockIdx.x] = a;
+    }
   }
+  __threadfence();
   __syncthreads();
-  if (threadIdx.x < nv) {
-    double acc = sh[0][threadIdx.x];
-    for (int w = 1; w < (int)(blockDim.x / 32); ++w)
-      acc = use_max ? fmax(acc, sh[w][threadIdx.x]) : acc + sh[w][threadIdx.x];
-    part[blockIdx.x * nv + threadIdx.x] = acc;
+  if (threadIdx.x == 0) last = atomicAdd(r.counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = wid; k < NV; k += kThreads / 32) {
+    const volatile double* p = r.part + (size_t)k * gridDim.x;
+    double a = lane < (int)gridDim.x ? p[lane] : (MAX ? -1.7e308 : 0.);
+    for (int b = lane + 32; b < (int)gridDim.x; b += 32) a = add(a, p[b]);
+    a = tree(a);
+    if (lane == 0) r.out[k] = a;
   }
+  if (threadIdx.x == 0) *r.counter = 0u;
 }
 
-__global__ void k_finish(const double* __restrict__ part, int nblk, int nv, double* __restrict__ out,
-                         int use_max) {
-  for (int k = threadIdx.x; k < nv; k += blockDim.x) {
-    double acc = part[k];
-    for (int b = 1; b < nblk; ++b) acc = use_max ? fmax(acc, part[b * nv + k]) : acc + part[b * nv + k];
-    out[k] = acc;
-  }
-}
-
-__global__ void k_sum(const double* __restrict__ v, long long n, double* part) {
+// The sum of a full field over the design box.
+__global__ void __launch_bounds__(kThreads) k_box_sum(Grid g, const int* __restrict__ b, long long n,
+                                                      const double* __restrict__ full,
+                                                      Reduction red) {
+  const int nxb = b[1] - b[0] + 1, nyb = b[3] - b[2] + 1;
   double acc[1] = {0.};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x)
-    acc[0] += v[i];
-  block_store(acc, 1, part, false);
+       i += (long long)gridDim.x * blockDim.x) {
+    const int x = (int)(i % nxb) + b[0];
+    const long long r = i / nxb;
+    const int y = (int)(r % nyb) + b[2];
+    const int z = (int)(r / nyb) + b[4];
+    acc[0] += full[((long long)z * g.ny + y) * g.nx + x];
+  }
+  grid_reduce_values<1, false>(acc, red);
 }
 
-__global__ void k_max_abs_diff(const double* __restrict__ a, const double* __restrict__ b,
-                               long long n, double* part) {
+__global__ void __launch_bounds__(kThreads) k_max_abs_diff(const double* __restrict__ a,
+                                                           const double* __restrict__ b,
+                                                           long long n, Reduction red) {
   double acc[1] = {0.};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x)
     acc[0] = fmax(acc[0], fabs(a[i] - b[i]));
-  block_store(acc, 1, part, true);
+  grid_reduce_values<1, true>(acc, red);
 }
 
 // ---------------------------------------------------------------------------
@@ -244,25 +326,28 @@ __global__ void k_max_abs_diff(const double* __restrict__ a, const double* __res
 
 struct MmaDev {
   long long n;
-  int m;
-  double *x, *x1, *x2, *L, *U, *al, *be, *p0, *q0, *P, *Q;   // P, Q: m x n
+  double *x, *x1, *x2, *L, *U, *al, *be, *p0, *q0;
+  double* G;            // m x n: P_ji where the derivative is positive, -Q_ji where negative
   const double* df0;
-  const double* dg;                                           // m x n
+  const double* dg;     // m x n
 };
 
 struct MmaScalars {
   int k;
   double asyminit, asymdec, asyminc, movlim;
   double lam[kMaxM];
-  int hess;
 };
 
 // Subproblem at the expansion point x (GenSub), the history shift, and the
-// block sums of sum_i (P_ji/(U-x) + Q_ji/(x-L)) for b_j.
-__global__ void k_mma_gensub(MmaDev d, MmaScalars s, double* part) {
+// sums of P_ji/(U-x) + Q_ji/(x-L) for b_j.  One of P_ji = (U-x)^2 max(0, g)
+// and Q_ji = (x-L)^2 max(0, -g) is zero, so one signed array holds both and
+// the quotients are (U-x) g or (x-L) (-g).
+template <int M>
+__global__ void __launch_bounds__(kThreads) k_mma_gensub(MmaDev d, MmaScalars s, Reduction red) {
   const double feps = 1.0e-6;
-  double acc[kMaxM];
-  for (int j = 0; j < d.m; ++j) acc[j] = 0.;
+  double acc[M];
+#pragma unroll
+  for (int j = 0; j < M; ++j) acc[j] = 0.;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < d.n;
        i += (long long)gridDim.x * blockDim.x) {
     const double x = d.x[i], x1 = d.x1[i], x2 = d.x2[i];
@@ -287,53 +372,85 @@ __global__ void k_mma_gensub(MmaDev d, MmaScalars s, double* part) {
     const double ux = U - x, xl = x - L, reg = 0.5 * feps / (U - L), df = d.df0[i];
     d.p0[i] = ux * ux * (fmax(0., df) + 0.001 * fabs(df) + reg);
     d.q0[i] = xl * xl * (fmax(0., -df) + 0.001 * fabs(df) + reg);
-    for (int j = 0; j < d.m; ++j) {
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
       const double gj = d.dg[(long long)j * d.n + i];
-      const double P = ux * ux * fmax(0., gj), Q = xl * xl * fmax(0., -gj);
-      d.P[(long long)j * d.n + i] = P;
-      d.Q[(long long)j * d.n + i] = Q;
-      acc[j] += P / ux + Q / xl;
+      const double h = gj > 0. ? ux : xl;
+      d.G[(long long)j * d.n + i] = h * h * gj;
+      acc[j] += h * fabs(gj);
     }
     d.x2[i] = x1;
     d.x1[i] = x;
   }
-  block_store(acc, d.m, part, false);
+  grid_reduce_values<M, false>(acc, red);
 }
 
-// x(lam) into d.x, and the block sums of the dual gradient terms and (hess)
-// of the dual Hessian's upper triangle.
-__global__ void k_mma_dual(MmaDev d, MmaScalars s, double* part) {
-  const int m = d.m;
-  const int nv = s.hess ? m + m * (m + 1) / 2 : m;
-  double acc[kMaxVals];
-  for (int k = 0; k < nv; ++k) acc[k] = 0.;
+// x(lam) into d.x, the sums of the dual gradient terms and of the dual
+// Hessian's upper triangle.  Bound by the FP64 pipe (two instructions per
+// clock and SM): two square roots, four quotients and about 60 other
+// operations per variable at M = 4, where the quotients P/(U-x), Q/(x-L),
+// P/(U-x)^2, Q/(x-L)^2 taken one by one cost some 20 divisions.
+template <int M>
+__global__ void __launch_bounds__(kThreads) k_mma_dual(MmaDev d, MmaScalars s, Reduction red) {
+  constexpr int NV = M + M * (M + 1) / 2;
+  double acc[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) acc[k] = 0.;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < d.n;
        i += (long long)gridDim.x * blockDim.x) {
-    double p = d.p0[i], q = d.q0[i];
-    for (int j = 0; j < m; ++j) {
-      p += d.P[(long long)j * d.n + i] * s.lam[j];
-      q += d.Q[(long long)j * d.n + i] * s.lam[j];
+    double p = d.p0[i], q = d.q0[i], G[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+      G[j] = d.G[(long long)j * d.n + i];
+      const bool pos = G[j] > 0.;
+      const double t = fma(fabs(G[j]), s.lam[j], pos ? p : q);
+      p = pos ? t : p;
+      q = pos ? q : t;
     }
-    const double L = d.L[i], U = d.U[i];
+    const double L = d.L[i], U = d.U[i], al = d.al[i], be = d.be[i];
     const double sp = sqrt(p), sq = sqrt(q);
     const double xf = (sp * L + sq * U) / (sp + sq);
-    const double x = fmin(fmax(xf, d.al[i]), d.be[i]);
+    const bool inside = !(xf < al || xf > be);
+    const double x = fmin(fmax(xf, al), be);
     d.x[i] = x;
-    const double ux = U - x, xl = x - L;
-    for (int j = 0; j < m; ++j)
-      acc[j] += d.P[(long long)j * d.n + i] / ux + d.Q[(long long)j * d.n + i] / xl;
-    if (s.hess && !(xf < d.al[i] || xf > d.be[i])) {
-      const double d2 = -1. / (2. * p / (ux * ux * ux) + 2. * q / (xl * xl * xl));
-      double pq[kMaxM];
-      for (int j = 0; j < m; ++j)
-        pq[j] = d.P[(long long)j * d.n + i] / (ux * ux) - d.Q[(long long)j * d.n + i] / (xl * xl);
-      int k = m;
-      for (int j = 0; j < m; ++j)
-        for (int l = j; l < m; ++l) acc[k++] += pq[j] * d2 * pq[l];
+    const double ru = 1. / (U - x), rl = 1. / (x - L);
+    double pq[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+      const double r = G[j] > 0. ? ru : rl, t = G[j] * r;
+      acc[j] += fabs(t);
+      pq[j] = t * r;
+    }
+    if (inside) {
+      const double d2 = -0.5 / (p * (ru * ru * ru) + q * (rl * rl * rl));
+      int k = M;
+#pragma unroll
+      for (int j = 0; j < M; ++j) {
+        const double t = pq[j] * d2;
+#pragma unroll
+        for (int l = j; l < M; ++l) acc[k++] += t * pq[l];
+      }
     }
   }
-  block_store(acc, nv, part, false);
+  grid_reduce_values<NV, false>(acc, red);
 }
+
+// f(std::integral_constant<int, m>) for the problem's number of constraints
+template <class F>
+void by_constraints(int m, F&& f) {
+  switch (m) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    default: f(std::integral_constant<int, 9>{}); break;
+  }
+}
+static_assert(kMaxM == 9, "by_constraints lists the numbers of constraints");
 
 void solve_small(double* A, double* r, int m) {
   for (int c = 0; c < m; ++c) {
@@ -364,6 +481,11 @@ int grid_for(long long n) {
   return (int)b;
 }
 
+int reduce_grid(long long n) {
+  const int b = grid_for(n);
+  return b < kReduceBlocks ? b : kReduceBlocks;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -379,6 +501,7 @@ struct lbm_topopt {
   struct Stage {
     int radius = 0, ntaps = 0;
     int* tap = nullptr;
+    long long* off = nullptr;
     double* w = nullptr;
     double* den = nullptr;
   } stage[LBM_MAX_STAGES];
@@ -389,9 +512,11 @@ struct lbm_topopt {
   bool have_sens[LBM_MAX_REALISATIONS] = {};
   // MMA
   double *x = nullptr, *x1 = nullptr, *x2 = nullptr, *L = nullptr, *U = nullptr, *al = nullptr,
-         *be = nullptr, *p0 = nullptr, *q0 = nullptr, *P = nullptr, *Q = nullptr, *df0 = nullptr,
-         *dg = nullptr, *zero = nullptr;
-  double *part = nullptr, *sums = nullptr;
+         *be = nullptr, *p0 = nullptr, *q0 = nullptr, *G = nullptr, *dg = nullptr, *zero = nullptr;
+  double* part = nullptr;
+  unsigned* counter = nullptr;
+  double* host = nullptr;          // results of the reductions (pinned, mapped)
+  double* host_dev = nullptr;      // its device address
   double a[kMaxM] = {}, c[kMaxM] = {};
   int k = 0;
   int dual_iterations = 0;
@@ -432,6 +557,8 @@ int talloc(lbm_topopt* t, double** p, long long count) {
 void tfree(lbm_topopt* t) {
   for (void* p : t->allocs) cudaFree(p);
   t->allocs.clear();
+  if (t->host) cudaFreeHost(t->host);
+  t->host = nullptr;
   if (t->st) cudaStreamDestroy(t->st);
   t->st = nullptr;
 }
@@ -446,12 +573,22 @@ StageDev stage_dev(const lbm_topopt* t, int k, int r) {
   for (int i = 0; i < 6; ++i) s.box[i] = c.filter_box[i];
   s.beta = c.beta[k];
   s.eta = (k == t->nstages - 1 && t->nreal > 1) ? c.real_eta[r] : c.eta[k];
-  s.pden = std::tanh(s.beta * s.eta) + std::tanh(s.beta * (1. - s.eta));
+  s.pnum = std::tanh(s.beta * s.eta);
+  s.pden = s.pnum + std::tanh(s.beta * (1. - s.eta));
+  s.reach = t->stage[k].radius - 1;   // taps lie closer than the radius
+  s.reach_z = t->g.nz > 1 ? s.reach : 0;
   s.tap = t->stage[k].tap;
+  s.off = t->stage[k].off;
   s.w = t->stage[k].w;
   s.den = t->stage[k].den;
   return s;
 }
+
+dim3 filter_grid(const Grid& g) {
+  const long long r = ((long long)g.ny * g.nz + kFilterY - 1) / kFilterY;
+  return dim3((g.nx + kFilterX - 1) / kFilterX, (unsigned)(r < 65535 ? r : 65535));
+}
+const dim3 kFilterBlock(kFilterX, kFilterY);
 
 int check_launch(lbm_topopt* t) {
   cudaError_t e = cudaGetLastError();
@@ -470,7 +607,8 @@ int forward_chain(lbm_topopt* t, int r) {
   }
   for (int k = 0; k < t->nstages; ++k) {
     double* out = (k == t->nstages - 1) ? t->gamma[r] : t->tmp2;
-    k_stage_forward<<<gb, kThreads, 0, t->st>>>(t->g, stage_dev(t, k, r), in, t->keep[r][k], out);
+    k_stage_forward<<<filter_grid(t->g), kFilterBlock, 0, t->st>>>(t->g, stage_dev(t, k, r), in,
+                                                                   t->keep[r][k], out);
     in = out;
   }
   return check_launch(t);
@@ -478,22 +616,23 @@ int forward_chain(lbm_topopt* t, int r) {
 
 // design sensitivity (n) from a full-grid sensitivity in t->tmp, realisation r
 int transpose_chain(lbm_topopt* t, int r, double* out_design) {
-  const int gb = grid_for(t->g.n);
+  const dim3 gb = filter_grid(t->g);
   for (int k = t->nstages - 1; k >= 0; --k) {
     StageDev s = stage_dev(t, k, r);
-    k_stage_scale<<<gb, kThreads, 0, t->st>>>(t->g, s, t->keep[r][k], t->tmp, t->tmp2);
-    k_stage_transpose<<<gb, kThreads, 0, t->st>>>(t->g, s, t->tmp2, t->tmp);
+    k_stage_scale<<<gb, kFilterBlock, 0, t->st>>>(t->g, s, t->keep[r][k], t->tmp, t->tmp2);
+    k_stage_transpose<<<gb, kFilterBlock, 0, t->st>>>(t->g, s, t->tmp2, t->tmp);
   }
   k_gather_box<<<grid_for(t->n), kThreads, 0, t->st>>>(t->g, t->box_d, t->n, t->tmp, out_design);
   return check_launch(t);
 }
 
-// fixed-order sum (or max) into host values
-int reduce_to_host(lbm_topopt* t, int nblk, int nv, bool use_max, double* host) {
-  k_finish<<<1, 64, 0, t->st>>>(t->part, nblk, nv, t->sums, use_max ? 1 : 0);
+Reduction reduction(const lbm_topopt* t) { return Reduction{t->part, t->counter, t->host_dev}; }
+
+// the nv results of the last reducing kernel
+int reduced(lbm_topopt* t, int nv, double* out) {
   TCUDA(t, cudaGetLastError());
-  TCUDA(t, cudaMemcpyAsync(host, t->sums, sizeof(double) * nv, cudaMemcpyDeviceToHost, t->st));
   TCUDA(t, cudaStreamSynchronize(t->st));
+  for (int k = 0; k < nv; ++k) out[k] = t->host[k];
   return 0;
 }
 
@@ -586,18 +725,35 @@ int lbm_topopt_create(const lbm_topopt_config* cfg, const double* background, co
   if ((rc = talloc(t, &t->bg, N)) || (rc = talloc(t, &t->xfull, N)) || (rc = talloc(t, &t->tmp, N)) ||
       (rc = talloc(t, &t->tmp2, N)))
     return bail(rc);
+  // the derivatives of several realisations are the first rows of the
+  // constraints' derivatives
+  if ((rc = talloc(t, &t->dg, (long long)t->m * n))) return bail(rc);
   for (int r = 0; r < t->nreal; ++r) {
-    if ((rc = talloc(t, &t->gamma[r], N)) || (rc = talloc(t, &t->df[r], n))) return bail(rc);
+    if ((rc = talloc(t, &t->gamma[r], N))) return bail(rc);
+    if (t->nreal > 1)
+      t->df[r] = t->dg + (long long)r * n;
+    else if ((rc = talloc(t, &t->df[r], n)))
+      return bail(rc);
     for (int k = 0; k < t->nstages; ++k)
       if ((rc = talloc(t, &t->keep[r][k], N))) return bail(rc);
   }
-  double** mm[] = {&t->x, &t->x1, &t->x2, &t->L, &t->U, &t->al, &t->be, &t->p0, &t->q0, &t->df0, &t->zero};
+  double** mm[] = {&t->x, &t->x1, &t->x2, &t->L, &t->U, &t->al, &t->be, &t->p0, &t->q0, &t->zero};
   for (double** p : mm)
     if ((rc = talloc(t, p, n))) return bail(rc);
-  if ((rc = talloc(t, &t->P, (long long)t->m * n)) || (rc = talloc(t, &t->Q, (long long)t->m * n)) ||
-      (rc = talloc(t, &t->dg, (long long)t->m * n)) ||
-      (rc = talloc(t, &t->part, (long long)kMaxBlocks * kMaxVals)) || (rc = talloc(t, &t->sums, kMaxVals)))
+  if ((rc = talloc(t, &t->G, (long long)t->m * n)) ||
+      (rc = talloc(t, &t->part, (long long)kReduceBlocks * kMaxVals)))
     return bail(rc);
+  if (cudaMalloc((void**)&t->counter, sizeof(unsigned)) != cudaSuccess) {
+    t->err = "cudaMalloc failed";
+    return bail(LBM_ERR_MEM);
+  }
+  t->allocs.push_back(t->counter);
+  cudaMemsetAsync(t->counter, 0, sizeof(unsigned), t->st);
+  if (cudaHostAlloc((void**)&t->host, kMaxVals * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&t->host_dev, t->host, 0) != cudaSuccess) {
+    t->err = "cudaHostAlloc failed";
+    return bail(LBM_ERR_MEM);
+  }
   int* bx = nullptr;
   if (cudaMalloc((void**)&bx, 6 * sizeof(int)) != cudaSuccess) {
     t->err = "cudaMalloc failed";
@@ -639,6 +795,7 @@ int lbm_topopt_create(const lbm_topopt_config* cfg, const double* background, co
   for (int k = 0; k < t->nstages; ++k) {
     const int R = c.radius[k], R3 = c.nz > 1 ? R : 0;
     std::vector<int> taps;
+    std::vector<long long> off;
     std::vector<double> w;
     for (int dz = -R3; dz <= R3; ++dz)
       for (int dy = -R; dy <= R; ++dy)
@@ -648,6 +805,7 @@ int lbm_topopt_create(const lbm_topopt_config* cfg, const double* background, co
             taps.push_back(dx);
             taps.push_back(dy);
             taps.push_back(dz);
+            off.push_back(((long long)dz * c.ny + dy) * c.nx + dx);
             w.push_back((double)R - d);
           }
         }
@@ -661,6 +819,14 @@ int lbm_topopt_create(const lbm_topopt_config* cfg, const double* background, co
     }
     t->allocs.push_back(tp);
     s.tap = tp;
+    long long* op = nullptr;
+    if (cudaMalloc((void**)&op, sizeof(long long) * off.size()) != cudaSuccess) {
+      t->err = "cudaMalloc failed";
+      return bail(LBM_ERR_MEM);
+    }
+    t->allocs.push_back(op);
+    s.off = op;
+    cudaMemcpyAsync(s.off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice, t->st);
     if ((rc = talloc(t, &s.w, (long long)w.size())) || (rc = talloc(t, &s.den, N))) return bail(rc);
     cudaMemcpyAsync(s.tap, taps.data(), sizeof(int) * taps.size(), cudaMemcpyHostToDevice, t->st);
     cudaMemcpyAsync(s.w, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice, t->st);
@@ -806,21 +972,16 @@ int lbm_topopt_update(lbm_topopt* t, double* change, double* constraints) {
   int j = 0;
   if (t->nreal > 1)
     for (int r = 0; r < t->nreal; ++r, ++j) {
-      g[j] = t->J[r] + c.magic;
-      TCUDA(t, cudaMemcpyAsync(t->dg + (long long)j * n, t->df[r], sizeof(double) * n,
-                               cudaMemcpyDeviceToDevice, t->st));
+      g[j] = t->J[r] + c.magic;   // its derivative is already in row j of dg
     }
   if (c.volume_type != LBM_VOLUME_NONE) {
     const int vr = c.volume_real;
     if ((rc = forward_chain(t, vr))) return rc;
     // mean of the physical field over the design box
     double* row = t->dg + (long long)j * n;
-    k_gather_box<<<grid_for(n), kThreads, 0, t->st>>>(t->g, t->box_d, n, t->gamma[vr], row);
-    const int nb = grid_for(n);
-    k_sum<<<nb, kThreads, 0, t->st>>>(row, n, t->part);
-    if ((rc = check_launch(t))) return rc;
+    k_box_sum<<<reduce_grid(n), kThreads, 0, t->st>>>(t->g, t->box_d, n, t->gamma[vr], reduction(t));
     double sum = 0.;
-    if ((rc = reduce_to_host(t, nb, 1, false, &sum))) return rc;
+    if ((rc = reduced(t, 1, &sum))) return rc;
     const double mean = sum / (double)n;
     g[j] = c.volume_type == LBM_VOLUME_FLUID ? -c.volume + mean : (1. - c.volume) - mean;
     // its sensitivity: +-1/n on the full grid, through the filters, onto the box
@@ -836,7 +997,7 @@ int lbm_topopt_update(lbm_topopt* t, double* change, double* constraints) {
   const double* df0 = t->nreal > 1 ? t->zero : t->df[0];
   // ---- MMA ----
   t->k += 1;
-  MmaDev d{n, m, t->x, t->x1, t->x2, t->L, t->U, t->al, t->be, t->p0, t->q0, t->P, t->Q, df0, t->dg};
+  MmaDev d{n, t->x, t->x1, t->x2, t->L, t->U, t->al, t->be, t->p0, t->q0, t->G, df0, t->dg};
   MmaScalars s;
   memset(&s, 0, sizeof(s));
   s.k = t->k;
@@ -844,11 +1005,13 @@ int lbm_topopt_update(lbm_topopt* t, double* change, double* constraints) {
   s.asymdec = 0.7;
   s.asyminc = 1.2;
   s.movlim = c.move_limit;
-  const int nb = grid_for(n);
+  const int nb = reduce_grid(n);
+  const Reduction red = reduction(t);
   double b[kMaxM];
-  k_mma_gensub<<<nb, kThreads, 0, t->st>>>(d, s, t->part);
-  if ((rc = check_launch(t))) return rc;
-  if ((rc = reduce_to_host(t, nb, m, false, b))) return rc;
+  by_constraints(m, [&](auto M) {
+    k_mma_gensub<decltype(M)::value><<<nb, kThreads, 0, t->st>>>(d, s, red);
+  });
+  if ((rc = reduced(t, m, b))) return rc;
   for (int i = 0; i < m; ++i) b[i] -= g[i];
 
   double lam[kMaxM], mu[kMaxM], vals[kMaxVals], gr[kMaxM], H[kMaxM * kMaxM], ds[kMaxM], dm[kMaxM];
@@ -856,47 +1019,45 @@ int lbm_topopt_update(lbm_topopt* t, double* change, double* constraints) {
     lam[i] = t->c[i] / 2.;
     mu[i] = 1.;
   }
-  // x(lam) on the device, y(lam), z(lam) and the dual gradient here
-  auto evaluate = [&](bool hess) -> int {
+  // x(lam) on the device, y(lam), z(lam), the dual gradient and Hessian here:
+  // both at once, as the next Newton step starts where the last one ended
+  auto evaluate = [&]() -> int {
     for (int i = 0; i < m; ++i) {
       if (lam[i] < 0.) lam[i] = 0.;
       s.lam[i] = lam[i];
     }
-    s.hess = hess ? 1 : 0;
-    k_mma_dual<<<nb, kThreads, 0, t->st>>>(d, s, t->part);
-    int r2 = check_launch(t);
-    if (r2) return r2;
-    const int nv = hess ? m + m * (m + 1) / 2 : m;
-    if ((r2 = reduce_to_host(t, nb, nv, false, vals))) return r2;
+    by_constraints(m, [&](auto M) {
+      k_mma_dual<decltype(M)::value><<<nb, kThreads, 0, t->st>>>(d, s, red);
+    });
+    int r2;
+    if ((r2 = reduced(t, m + m * (m + 1) / 2, vals))) return r2;
     double la = 0.;
     for (int i = 0; i < m; ++i) la += lam[i] * t->a[i];
     const double z = std::max(0., 10. * (la - 1.));
     for (int i = 0; i < m; ++i) gr[i] = vals[i] - b[i] - t->a[i] * z - std::max(0., lam[i] - t->c[i]);
-    if (hess) {
-      int k = m;
+    int k = m;
+    for (int i = 0; i < m; ++i)
+      for (int l = i; l < m; ++l) {
+        H[i * m + l] = vals[k];
+        H[l * m + i] = vals[k];
+        ++k;
+      }
+    for (int i = 0; i < m; ++i)
+      if (lam[i] > t->c[i]) H[i * m + i] -= 1.;
+    if (la > 1.)
       for (int i = 0; i < m; ++i)
-        for (int l = i; l < m; ++l) {
-          H[i * m + l] = vals[k];
-          H[l * m + i] = vals[k];
-          ++k;
-        }
-      for (int i = 0; i < m; ++i)
-        if (lam[i] > t->c[i]) H[i * m + i] -= 1.;
-      if (la > 1.)
-        for (int i = 0; i < m; ++i)
-          for (int l = 0; l < m; ++l) H[i * m + l] -= 10. * t->a[i] * t->a[l];
-    }
+        for (int l = 0; l < m; ++l) H[i * m + l] -= 10. * t->a[i] * t->a[l];
     return 0;
   };
   const double tol = 1.0e-9 * std::sqrt((double)(m + n));
   double eps = 1., err = 1.;
   int iters = 0;
+  if ((rc = evaluate())) return rc;
   while (eps > tol) {
     int loop = 0;
     while (err > 0.9 * eps && loop < 100) {
       ++loop;
       ++iters;
-      if ((rc = evaluate(true))) return rc;
       double tr = 0.;
       for (int i = 0; i < m; ++i) {
         H[i * m + i] -= mu[i] / lam[i];
@@ -919,7 +1080,7 @@ int lbm_topopt_update(lbm_topopt* t, double* change, double* constraints) {
         lam[i] += th * ds[i];
         mu[i] += th * dm[i];
       }
-      if ((rc = evaluate(false))) return rc;
+      if ((rc = evaluate())) return rc;
       err = 0.;
       for (int i = 0; i < m; ++i) {
         err = std::max(err, std::fabs(gr[i] + mu[i]));
@@ -930,10 +1091,9 @@ int lbm_topopt_update(lbm_topopt* t, double* change, double* constraints) {
   }
   t->dual_iterations = iters;
   // x now holds x(lam); the change against the expansion point
-  k_max_abs_diff<<<nb, kThreads, 0, t->st>>>(t->x, t->x1, n, t->part);
-  if ((rc = check_launch(t))) return rc;
+  k_max_abs_diff<<<nb, kThreads, 0, t->st>>>(t->x, t->x1, n, red);
   double ch = 0.;
-  if ((rc = reduce_to_host(t, nb, 1, true, &ch))) return rc;
+  if ((rc = reduced(t, 1, &ch))) return rc;
   if (change) *change = ch;
   if (constraints)
     for (int i = 0; i < m; ++i) constraints[i] = g[i];
