@@ -66,6 +66,11 @@ inline FixedModel fixed_model(const lbm_config& c) {
   }
   // (9/2) nu omega^2 = (3/2) omega (1 - omega/2), at most 3/4
   m.cv = fixed_constant(1.5L * om * (1 - om / 2), 64, ok);
+  const long double w = frexpl(fabsl((long double)c.obj_weight), &m.w_exp);
+  bool weight = true;
+  m.w = fixed_constant(w, 64, weight);
+  m.w_neg = c.obj_weight < 0. ? -1 : 0;
+  if (!weight) ok = ok && c.objective != LBM_OBJ_DISSIPATION;
   m.ok = ok ? 1 : 0;
   return m;
 }

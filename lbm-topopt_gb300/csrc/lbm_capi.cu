@@ -158,6 +158,7 @@ struct lbm_handle {
   Geometry geo_fwd;   // forward step (autotuned)
   Geometry geo_adj;   // reverse step (autotuned)
   bool adj_lean = false;   // reverse step: the register-lean variant (autotuned)
+  bool adj_wide = false;   // FP64 D2Q9 reverse step with three resident blocks (wide_reverse)
   bool sens_atomic = false;   // reverse step adds to dJ/dgamma atomically (fits in L2)
   bool tuned = false;
   size_t partial_cap = 0;
@@ -268,6 +269,18 @@ bool fits_in_l2(size_t bytes) {
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) return false;
   return bytes <= (size_t)l2;
+}
+
+// Whether the reverse steps of a lattice (or batch) of that many cells run with
+// one more resident block per SM by default: FP64 D2Q9 lattices past one wave
+// of two 256-thread blocks per SM (see Occupancy in lbm_kernels.cuh).
+bool wide_reverse(const lbm_config& c, int64_t ncell) {
+  int dev = 0, nsm = 0;
+  if (c.storage != LBM_STORE_FP64 || c.lattice != LBM_D2Q9) return false;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  return ncell > (int64_t)nsm * 512;
 }
 
 int check_box(const lbm_config& c, const int* b, int dim, const char* what) {
@@ -613,7 +626,7 @@ int adjoint_at(lbm_handle* h, const void* f) {
   p.lam_in = h->lam[h->lcur];
   p.lam_out = h->lam[1 - h->lcur];
   p.eval_obj = (h->t >= h->obj_from && h->cfg.objective != LBM_OBJ_NONE) ? 1 : 0;
-  int rc = launch(h, h->adj_lean ? K_ADJOINT_LEAN : K_ADJOINT, p, nullptr);
+  int rc = launch(h, h->adj_lean || h->adj_wide ? K_ADJOINT_LEAN : K_ADJOINT, p, nullptr);
   if (rc) return rc;
   h->lcur ^= 1;
   return 0;
@@ -761,6 +774,7 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   h->adj_bytes = c.storage == LBM_STORE_FP64 ? 8 : 4;
   h->gam_bytes = c.storage == LBM_STORE_FP64 ? 8 : 4;
   h->sens_atomic = fits_in_l2(reverse_step_bytes(h));
+  h->adj_wide = wide_reverse(c, h->ncell);
   h->launch = c.lattice == LBM_D2Q9    ? launcher_d2q9(c.collision, c.storage)
               : c.lattice == LBM_D3Q19 ? launcher_d3q19(c.collision, c.storage)
                                        : launcher_thermal(c.collision, c.storage);
@@ -1594,6 +1608,7 @@ struct lbm_batch {
   int bx = 128, by = 2;     // block shape of the forward and objective kernels
   int abx = 128, aby = 2;   // block shape of the reverse step kernel
   bool adj_lean = false;    // reverse step: the register-lean variant
+  bool adj_wide = false;    // its default for FP64 D2Q9 (see lbm_handle)
   bool sens_atomic = false; // the batched reverse step fits in L2 (see lbm_handle)
   int nsm = 1;
   int grid_fwd = 1, grid_adj = 1, grid_obj = 1, grid_copy = 1;
@@ -1687,7 +1702,8 @@ void batch_set_grids(lbm_batch* b) {
   batch_layout(b, bp, K_OBJECTIVE);
   b->grid_obj = batch_grid(b, K_OBJECTIVE, bp.start[b->n]);
   batch_layout(b, bp, K_ADJOINT);
-  b->grid_adj = batch_grid(b, b->adj_lean ? K_ADJOINT_LEAN : K_ADJOINT, bp.start[b->n]);
+  b->grid_adj =
+      batch_grid(b, b->adj_lean || b->adj_wide ? K_ADJOINT_LEAN : K_ADJOINT, bp.start[b->n]);
 }
 
 int batch_launch(lbm_batch* b, int kind, const BatchParams& bp, int grid) {
@@ -1767,7 +1783,7 @@ int batch_adjoint(lbm_batch* b, int buf) {
     p.eval_obj = (h->t >= 1 && h->cfg.objective != LBM_OBJ_NONE) ? 1 : 0;
     p.sens_atomic = b->sens_atomic ? 1 : 0;
   }
-  int rc = batch_launch(b, b->adj_lean ? K_ADJOINT_LEAN : K_ADJOINT, bp, b->grid_adj);
+  int rc = batch_launch(b, b->adj_lean || b->adj_wide ? K_ADJOINT_LEAN : K_ADJOINT, bp, b->grid_adj);
   if (rc) return rc;
   for (int i = 0; i < b->n; ++i) b->h[i]->lcur ^= 1;
   return 0;
@@ -1955,7 +1971,12 @@ int lbm_batch_create(const lbm_config* cfgs, int n, lbm_batch** out) {
   batch_set_grids(b);
   b->grid_copy = 4 * b->nsm;
   size_t rev = 0;
-  for (int i = 0; i < b->n; ++i) rev += reverse_step_bytes(b->h[i]);
+  int64_t cells = 0;
+  for (int i = 0; i < b->n; ++i) {
+    rev += reverse_step_bytes(b->h[i]);
+    cells += b->h[i]->ncell;
+  }
+  b->adj_wide = wide_reverse(cfgs[0], cells);
   b->sens_atomic = fits_in_l2(rev);
   *out = b;
   return LBM_OK;

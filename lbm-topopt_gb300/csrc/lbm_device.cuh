@@ -259,6 +259,9 @@ struct FixedModel {
   unsigned long long c[12];          // factors below 1, times 2^64
   unsigned long long wej, wxx, we3c; // |wej/4|, |wxx| and |(we - 3)/4| times 2^62
   unsigned long long cv;             // the dissipation's viscous factor (9/2) nu omega^2 times 2^64
+  // the objective weight, |w| = w 2^(w_exp - 64) with its sign (0 or -1)
+  unsigned long long w;
+  int w_exp, w_neg;
 };
 
 struct KParams {

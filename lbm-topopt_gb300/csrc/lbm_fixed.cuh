@@ -299,36 +299,49 @@ __device__ __forceinline__ void mrt3d_collide(const i64* x, const Factor& im, co
 // of an FP64 sum over the cell; the derivative by imult takes the differences
 // as they are.
 
-struct Block {
-  int k = 0;       // values * 2^k
+template <int BITS>
+struct BlockOf {
+  int k = 0;       // values * 2^k, the largest below 2^BITS
+  int top = 0;     // exponent field of the largest
   bool zero = false, ok = false;
   // scale from the largest magnitude; exponents past these bounds (1e-210,
   // 1e16) and values that are not finite are left to the FP64 operators.
   // zero: no adjoint has arrived at the cell yet, and the transposed
   // collision, which is linear, leaves it so.
-  template <int N, int BITS = 60>
+  template <int N>
   __device__ __forceinline__ void measure(const double* v) {
     u32 m = 0u;
     static_for<N>([&](auto Q_) {
       const u32 h = hi_word(v[decltype(Q_)::value]) & 0x7fffffffu;
       m = h > m ? h : m;
     });
-    int e = (int)(m >> 20);
+    top = (int)(m >> 20);
     zero = m == 0u;
-    ok = e >= 323 && e <= 1077;
-    k = 1022 + BITS - e;
+    ok = top >= 323 && top <= 1077;
+    k = 1022 + BITS - top;
   }
+  // v * 2^k rounded to the nearest integer.  The conversion runs on the FP64
+  // pipe, except that the temperature lattice, whose two scales and FP64 terms
+  // keep that pipe busy, builds the integer from the words (512x256 step 11.4
+  // -> 10.3 us forward, 24.3 -> 23.4 us reverse; the D3Q19 reverse step, short
+  // of registers, went 0.515 -> 0.536 ms with it).
   __device__ __forceinline__ i64 load(double v) const {
-    const double d = from_words(hi_word(v) + ((u32)k << 20), lo_word(v));
 #if defined(__CUDA_ARCH__)
-    return __double2ll_rn(d);
-#else
-    return (i64)nearbyint(d);
+    if constexpr (BITS == 60) {
+      return __double2ll_rn(from_words(hi_word(v) + ((u32)k << 20), lo_word(v)));
+    }
 #endif
+    const u32 h = hi_word(v);
+    const int sh = top - (int)((h >> 20) & 0x7ffu);   // below the largest by 2^sh
+    const u64 m = ((u64)((h & 0xfffffu) | 0x100000u) << 32 | lo_word(v)) << (BITS - 52);
+    const i64 a = (i64)(((m >> (sh < 63 ? sh : 63)) + 1u) >> 1);
+    const i64 s = (i64)((int)h >> 31);
+    return (a ^ s) - s;
   }
   // results: 2 lam at the reduced scale
   __device__ __forceinline__ double store(i64 v) const { return to_double(v, k - 3); }
 };
+using Block = BlockOf<60>;
 
 // -sum a * w over the pairs, a * 2^61 and w in a Block's units (|a| < 0.6, |w|
 // < 2^61): products of 31-bit limbs, exact to 2^-86 of the largest.
@@ -519,11 +532,29 @@ __device__ __forceinline__ double load2(const double* lam, const Block& b, const
   return rev.value(b);
 }
 
+// What an objective adds to the adjoint of a 2D cell, in the units of
+// Block::store: ev[k] to both populations of pair k (ev[0] to the rest one)
+// and +-e_k . (gx, gy) to them.
+struct Source2 {
+  bool on = false;
+  i64 ev[5], gx, gy;
+  __device__ __forceinline__ void add(i64* S, i64* F, i64& f0) const {
+    if (!on) return;
+    f0 += ev[0];
+    static_for<4>([&](auto D) {
+      constexpr int k = decltype(D)::value + 1;
+      S[k] += ev[k];
+      F[k] += e_dot<LAT_D2Q9, k>(gx, gy, (i64)0);
+    });
+  }
+};
+
 // Transpose of bgk2_collide: lam + om (E^T lam - lam) with (E^T lam)_i = c0 +
 // e_i . c, 36 c0 = 16 lam_0 + (s1 + s3) + 4 (s2 + s4) and 12 c_x = (d1 - d3 -
 // 4 d4) + 2 jx (s1 + s3 + 4 s4 - 2 s2 - 8 lam_0) + 3 jy (s3 - s1) (y alike).
 __device__ __forceinline__ double bgk2_reverse(const i64* x, double* lam, const Block& b,
-                                               const Factor& im, const FixedModel& m) {
+                                               const Factor& im, const FixedModel& m,
+                                               const Source2& src) {
   const Pairs2 t(x);
   i64 o[5], ls[5], la[5];
   bgk2_odd(t, m, o);
@@ -549,7 +580,9 @@ __device__ __forceinline__ double bgk2_reverse(const i64* x, double* lam, const 
     F[k] = la[k] + mulc(ec, h6);
   });
   // 2 (lam_0 + om (c0 - lam_0))
-  store2(S, F, (v0 << 1) + mulc(c36 - 36 * v0, h18), b, lam);
+  i64 f0 = (v0 << 1) + mulc(c36 - 36 * v0, h18);
+  src.add(S, F, f0);
+  store2(S, F, f0, b, lam);
   return rev;
 }
 
@@ -593,7 +626,8 @@ __device__ __forceinline__ void mrt2_collide(const i64* x, const Factor& im, con
 }
 
 __device__ __forceinline__ double mrt2_reverse(const i64* x, double* lam, const Block& b,
-                                               const Factor& im, const FixedModel& m) {
+                                               const Factor& im, const FixedModel& m,
+                                               const Source2& src) {
   const Pairs2 t(x);
   i64 o[5], ls[5], la[5];
   mrt2_odd(t, m, o);
@@ -624,7 +658,9 @@ __device__ __forceinline__ double mrt2_reverse(const i64* x, double* lam, const 
   F[3] = la[3] - (dx + dy);
   F[2] = la[2] - (gy + n3);
   F[4] = la[4] - (gx + n2);
-  store2(S, F, (v0 << 1) + ((a8 + 1) >> 1) - (b1 << 1), b, lam);
+  i64 f0 = (v0 << 1) + ((a8 + 1) >> 1) - (b1 << 1);
+  src.add(S, F, f0);
+  store2(S, F, f0, b, lam);
   return rev;
 }
 
@@ -739,12 +775,12 @@ __device__ __forceinline__ double bgk3_reverse(const i64* x, double* lam, const 
 // populations are linear in it.  om6: om_T / 6 * 2^64.  The solid's heating
 // source is added in FP64, where there is any.
 
-constexpr int kThermalBits = 58;
+using ThermalBlock = BlockOf<58>;
 
 // T and 3 T u of the populations g (in a Block's units)
 struct Thermal {
   i64 g[5], T, tx, ty;
-  __device__ __forceinline__ Thermal(const double* gp, const Block& b, i64 jx, i64 jy) {
+  __device__ __forceinline__ Thermal(const double* gp, const ThermalBlock& b, i64 jx, i64 jy) {
     static_for<5>([&](auto I) { g[decltype(I)::value] = b.load(gp[decltype(I)::value]); });
     T = g[0] + ((g[1] + g[3]) + (g[2] + g[4]));
     tx = 3 * mulr(jx << 2, T << 1);
@@ -761,7 +797,7 @@ struct Thermal {
   }
 };
 
-__device__ __forceinline__ void thermal_collide(const Thermal& t, const Block& b, u64 om6,
+__device__ __forceinline__ void thermal_collide(const Thermal& t, const ThermalBlock& b, u64 om6,
                                                 double* gp) {
   i64 left = 0;
   static_for<4>([&](auto I) {
@@ -779,7 +815,7 @@ __device__ __forceinline__ void thermal_collide(const Thermal& t, const Block& b
 struct ThermalAdjoint {
   double dx, dy, sum6;
 };
-__device__ __forceinline__ ThermalAdjoint thermal_reverse(double* lam, const Block& l, i64 jx,
+__device__ __forceinline__ ThermalAdjoint thermal_reverse(double* lam, const ThermalBlock& l, i64 jx,
                                                           i64 jy, u64 om6) {
   i64 v[5];
   static_for<5>([&](auto I) { v[decltype(I)::value] = l.load(lam[decltype(I)::value]); });
@@ -827,30 +863,67 @@ __device__ __forceinline__ double dissipation2(const i64* x, u64 im, double w, d
   return w * (2. * (alpha * v.jj()) + cv * ((xx * xx + yy * yy) + 2. * (xy * xy)));
 }
 
-// lam += w dF/df, and the return value w dF/d(imult); c: cv * 2^64
-__device__ __forceinline__ double dissipation2_source(const i64* x, u64 im, double w, u64 c,
-                                                      double* lam) {
-  const Stress2 v(x, Pairs2(x));
-  constexpr u64 kThird = 0x5555555555555556ull;
-  const i64 t3 = mulc(v.xx + v.yy, kThird);
-  // V j
-  const i64 vx = mulr(v.qx, v.xx << 1) + mulr(v.qy, v.xy << 1);
-  const i64 vy = mulr(v.qx, v.xy << 1) + mulr(v.qy, v.yy << 1);
-  // 4 (alpha j - cv V j) along e, 2 cv (e.V e - tr/3) even
-  const i64 gx = mulc(v.qx, im) - (mulc(vx, c) << 2), gy = mulc(v.qy, im) - (mulc(vy, c) << 2);
-  const i64 d = v.xx + v.yy - t3, s = v.xy << 1;
-  const i64 ev[5] = {-(mulc(t3 << 1, c)), mulc((d - s) << 1, c), mulc((v.yy - t3) << 1, c),
-                     mulc((d + s) << 1, c), mulc((v.xx - t3) << 1, c)};
-  const double w61 = w * 4.336808689942017736029811203479766845703125e-19;   // w 2^-61
-  lam[0] += w61 * from_int(ev[0]);
-  static_for<4>([&](auto D) {
-    constexpr int k = decltype(D)::value + 1;
-    const i64 eg = e_dot<LAT_D2Q9, k>(gx, gy, (i64)0);
-    lam[k] += w61 * from_int(ev[k] + eg);
-    lam[k + 4] += w61 * from_int(ev[k] - eg);
-  });
-  return 2. * w * v.jj();
-}
+// The objective's derivatives by f and by imult, both over the weight.
+struct Dissipation2 {
+  Source2 src;    // * 2^61
+  double dim;     // 2 j^2
+  // c: cv * 2^64
+  __device__ __forceinline__ Dissipation2(const i64* x, const Factor& im, u64 c) {
+    const Stress2 v(x, Pairs2(x));
+    constexpr u64 kThird = 0x5555555555555556ull;
+    const i64 t3 = mulc(v.xx + v.yy, kThird);
+    // V j
+    const i64 vx = mulr(v.qx, v.xx << 1) + mulr(v.qy, v.xy << 1);
+    const i64 vy = mulr(v.qx, v.xy << 1) + mulr(v.qy, v.yy << 1);
+    // 4 (alpha j - cv V j) along e, 2 cv (e.V e - tr/3) even
+    src.gx = im.times(v.qx) - (mulc(vx, c) << 2);
+    src.gy = im.times(v.qy) - (mulc(vy, c) << 2);
+    const i64 d = v.xx + v.yy - t3, s = v.xy << 1;
+    src.ev[0] = -mulc(t3 << 1, c);
+    src.ev[1] = mulc((d - s) << 1, c);
+    src.ev[2] = mulc((v.yy - t3) << 1, c);
+    src.ev[3] = mulc((d + s) << 1, c);
+    src.ev[4] = mulc((v.xx - t3) << 1, c);
+    dim = 2. * v.jj();
+  }
+  // the source times the weight in the units of a Block's results, where that
+  // fits (on): it does unless the adjoint is much smaller than the weight, as
+  // in the first reverse steps
+  __device__ __forceinline__ Source2 scaled(const FixedModel& m, const Block& b) const {
+    Source2 r;
+    const int sh = m.w_exp + b.k - 64;
+    i64 v[7] = {src.ev[0], src.ev[1], src.ev[2], src.ev[3], src.ev[4], src.gx, src.gy};
+    u64 any = 0u;
+    static_for<7>([&](auto I) {
+      i64& t = v[decltype(I)::value];
+      t = mulc(t, m.w);
+      any |= (u64)(t ^ (t >> 63));
+    });
+    r.on = !b.zero && b.ok && sh < 28 && (sh <= 0 || (any >> (60 - sh)) == 0u);
+    const int l = sh > 0 ? sh : 0, q = sh < 0 ? (sh > -63 ? -sh : 63) : 0;
+    const i64 half = q > 0 ? 1ll << (q - 1) : 0, neg = m.w_neg;
+    static_for<7>([&](auto I) {
+      i64& t = v[decltype(I)::value];
+      t = ((t << l) + half) >> q;
+      t = (t ^ neg) - neg;
+    });
+    static_for<5>([&](auto I) { r.ev[decltype(I)::value] = v[decltype(I)::value]; });
+    r.gx = v[5];
+    r.gy = v[6];
+    return r;
+  }
+  // lam += w dF/df in FP64
+  __device__ __forceinline__ void add(double w, double* lam) const {
+    const double w61 = w * 4.336808689942017736029811203479766845703125e-19;   // w 2^-61
+    lam[0] += w61 * from_int(src.ev[0]);
+    static_for<4>([&](auto D) {
+      constexpr int k = decltype(D)::value + 1;
+      const i64 eg = e_dot<LAT_D2Q9, k>(src.gx, src.gy, (i64)0);
+      lam[k] += w61 * from_int(src.ev[k] + eg);
+      lam[k + 4] += w61 * from_int(src.ev[k] - eg);
+    });
+  }
+};
 
 // f <- the flow collision of LAT and COLL.
 template <int LAT, int COLL>
@@ -862,14 +935,16 @@ __device__ __forceinline__ void collide(const i64* x, const Factor& im, const Fi
   if constexpr (LAT == LAT_D2Q9 && COLL == LBM_MRT) mrt2_collide(x, im, m, f);
 }
 
-// lam <- its transpose; returns the derivative by imult.
+// lam <- its transpose (plus src on the 2D lattices); returns the derivative by
+// imult.
 template <int LAT, int COLL>
 __device__ __forceinline__ double reverse(const i64* x, double* lam, const Block& b,
-                                          const Factor& im, const FixedModel& m) {
+                                          const Factor& im, const FixedModel& m,
+                                          const Source2& src) {
   if constexpr (LAT == LAT_D3Q19 && COLL == LBM_MRT) return mrt3d_reverse(x, lam, b, im, m);
   if constexpr (LAT == LAT_D3Q19 && COLL == LBM_BGK) return bgk3_reverse(x, lam, b, im, m);
-  if constexpr (LAT != LAT_D3Q19 && COLL == LBM_BGK) return bgk2_reverse(x, lam, b, im, m);
-  if constexpr (LAT == LAT_D2Q9 && COLL == LBM_MRT) return mrt2_reverse(x, lam, b, im, m);
+  if constexpr (LAT != LAT_D3Q19 && COLL == LBM_BGK) return bgk2_reverse(x, lam, b, im, m, src);
+  if constexpr (LAT == LAT_D2Q9 && COLL == LBM_MRT) return mrt2_reverse(x, lam, b, im, m, src);
 }
 
 }  // namespace fx

@@ -43,11 +43,18 @@ struct Occupancy {
   static constexpr int adj_lean_batch = (LAT == LAT_D2Q9) ? adj + 2 : adj + 1;
   static constexpr bool has_lean = true;
 };
+// FP64 storage, whose collisions run on the integer pipes: 3 blocks (85
+// registers) of the D2Q9 forward step and 2 (128) of the others keep enough
+// warps in flight (at 190 registers the D3Q19 reverse step had 7.5 warps per
+// SM and took 0.731 ms on 256x128x128 against 0.515).  The D2Q9 reverse step
+// takes 2 where the lattice fits the SMs in one wave of them, and 3 on larger
+// ones (wide_reverse in lbm_capi.cu): 4096x2048 0.332 -> 0.294 ms, 1024x512 with
+// dissipation 43.9 -> 41.1 us, but 128x64 6.2 -> 6.7 us and 201x201 7.8 -> 8.4 us.
 template <int LAT, int COLL>
 struct Occupancy<LAT, COLL, double> {
   static constexpr int fwd = LAT == LAT_D2Q9 ? 3 : 2, adj = 2;
-  static constexpr int adj_lean = adj, adj_lean_batch = adj;
-  static constexpr bool has_lean = false;
+  static constexpr int adj_lean = LAT == LAT_D2Q9 ? 3 : 2, adj_lean_batch = adj_lean;
+  static constexpr bool has_lean = LAT == LAT_D2Q9;
 };
 
 template <class S>
@@ -295,6 +302,12 @@ __device__ __noinline__ void reverse_fp64(const double* f, double* lam, double g
   }
 }
 
+// The dissipation's source onto the adjoint of a cell whose units do not take it.
+static __device__ __noinline__ void add_dissipation_fp64(const fx::i64* x, unsigned long long im,
+                                                  const KParams& p, double* lam) {
+  fx::Dissipation2(x, fx::Factor(im), p.fix.cv).add(p.md.obj_weight, lam);
+}
+
 // Whether the collision runs in fixed point: FP64 storage.
 template <class S>
 constexpr bool kFixed = std::is_same<S, double>::value;
@@ -335,9 +348,9 @@ __device__ __forceinline__ double forward_cell_fixed(const KParams& p, int x, in
   });
   bool ok = w.template ok<LAT>(xi) && des.ok();
   if (p.fix.rest) ok = ok && !fx::at_rest<LAT>(xi);
-  fx::Block bt;
+  fx::ThermalBlock bt;
   if constexpr (THERMAL) {
-    bt.template measure<5, fx::kThermalBits>(f + 9);
+    bt.template measure<5>(f + 9);
     ok = ok && (bt.zero || bt.ok);
   }
   if (ok) {
@@ -417,7 +430,8 @@ __device__ __forceinline__ void add_sensitivity(double* sens, int c, double dg, 
 // of dJ/dgamma.  g, l: scales of the cell's temperatures and of their adjoint.
 __device__ __forceinline__ double thermal_reverse_cell(const KParams& p, int c, const double* f,
                                                        double* lam, const fx::Pairs2& u,
-                                                       const fx::Block& g, const fx::Block& l,
+                                                       const fx::ThermalBlock& g,
+                                                       const fx::ThermalBlock& l,
                                                        unsigned long long om6) {
   double dg = 0., T = 0.;
   if (!g.zero) {
@@ -463,12 +477,13 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
   const double dimult = p.dimult[c];
   if (on_bc_face<LAT>(x, y, p)) apply_bcs<LAT, false>(f, x, y, z, p);
   double dg = 0.;
-  fx::Block b, l, g;
+  fx::Block b;
+  fx::ThermalBlock l, g;
   b.template measure<L::QF>(lam);
   bool zero = b.zero, ok = b.zero || b.ok;
   if constexpr (THERMAL) {
-    l.template measure<5, fx::kThermalBits>(lam + 9);
-    g.template measure<5, fx::kThermalBits>(f + 9);
+    l.template measure<5>(lam + 9);
+    g.template measure<5>(f + 9);
     zero = zero && l.zero;
     ok = ok && (l.zero || l.ok) && (g.zero || g.ok);
   }
@@ -484,13 +499,35 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
     ok = ok && w.template ok<LAT>(xi) && des.ok();
     if (p.fix.rest) ok = ok && !fx::at_rest<LAT>(xi);
     if (ok) {
-      if (!b.zero) dg = dimult * fx::reverse<LAT, COLL>(xi, lam, b, fx::Factor(des.im), p.fix);
+      const fx::Factor im(des.im);
+      fx::Source2 src;
+      double ddiss = 0.;
+      if constexpr (L::DIM == 2) {
+        if (diss) {
+          const fx::Dissipation2 d(xi, im, p.fix.cv);
+          src = d.scaled(p.fix, b);
+          ddiss = dimult * (p.md.obj_weight * d.dim);
+        }
+      }
+      if (!b.zero) dg = dimult * fx::reverse<LAT, COLL>(xi, lam, b, im, p.fix, src);
       if constexpr (THERMAL) {
         if (!l.zero) dg += thermal_reverse_cell(p, c, f, lam, fx::Pairs2(xi), g, l, des.om6);
       }
       if constexpr (L::DIM == 2) {
-        if (diss)
-          dg += dimult * fx::dissipation2_source(xi, des.im, p.md.obj_weight, p.fix.cv, lam);
+        if (diss) {
+          dg += ddiss;
+          if (!src.on) {
+            fx::i64 xs[L::QF];
+            double s[L::QF];
+            static_for<L::QF>([&](auto Q_) {
+              constexpr int q = decltype(Q_)::value;
+              xs[q] = xi[q];
+              s[q] = lam[q];
+            });
+            add_dissipation_fp64(xs, des.im, p, s);
+            static_for<L::QF>([&](auto Q_) { lam[decltype(Q_)::value] = s[decltype(Q_)::value]; });
+          }
+        }
       }
     } else {
       double t[L::Q], u[L::Q], d = 0.;

@@ -106,7 +106,7 @@ int transpose(const lbm_config* c, int n, const double* f, const double* g, cons
     } else if (w.template ok<LAT>(x) && b.ok) {
       memcpy(a, lo + i * Q, sizeof(a));
       dgf[i] = fx::reverse<LAT, COLL>(x, a, b, fx::Factor((fx::u64)(imult * 18446744073709551616.)),
-                                       p.fix);
+                                       p.fix, fx::Source2());
       ++taken;
     }
     memcpy(fixed + i * Q, a, sizeof(a));
@@ -157,9 +157,9 @@ int fixed_thermal(int n, const double* f, const double* t, const double* l, cons
     });
     if (!w.ok<LAT_D2Q9_D2Q5>(x)) return i;
     const fx::Pairs2 u(x);
-    fx::Block b, a;
-    b.measure<5, fx::kThermalBits>(t + 5 * i);
-    a.measure<5, fx::kThermalBits>(l + 5 * i);
+    fx::ThermalBlock b, a;
+    b.measure<5>(t + 5 * i);
+    a.measure<5>(l + 5 * i);
     const fx::u64 om6 = (fx::u64)(om[i] * 3074457345618258602.7);
     memcpy(out + 5 * i, t + 5 * i, 40);
     memcpy(lout + 5 * i, l + 5 * i, 40);
@@ -185,12 +185,14 @@ int fixed_thermal(int n, const double* f, const double* t, const double* l, cons
   return n;
 }
 
-// Dissipation of n cells (weight 1): value, source (n x 9) and derivative by
-// imult, in fixed point and (value, source) by the objective functor.
+// Dissipation of n cells: value, source (n x 9) and derivative by imult (over
+// the weight), in fixed point and (value, source) by the objective functor;
+// scaled: the cells whose source fitted the adjoint's units.
 int fixed_dissipation(const lbm_config* c, int n, const double* f, const double* g, double* val,
-                      double* src, double* dim, double* val64, double* src64) {
+                      double* src, double* dim, double* val64, double* src64, int* scaled) {
   KParams p = params(c);
-  p.md.obj_weight = 1.;
+  p.md.obj_weight = c->obj_weight;
+  *scaled = 0;
   p.md.cv_diss = 4.5 * ((1. / c->omega - 0.5) / 3.) * c->omega * c->omega;
   for (int i = 0; i < n; ++i) {
     const double imult = 0.5 * (p.md.pbb_scale * bp(g[i], p.md.pbb_q));
@@ -202,9 +204,28 @@ int fixed_dissipation(const lbm_config* c, int n, const double* f, const double*
       x[q] = w.load<LAT_D2Q9, q>(f[i * 9 + q]);
     });
     if (!w.ok<LAT_D2Q9>(x)) return i;
-    val[i] = fx::dissipation2(x, im, 1., p.md.cv_diss);
+    val[i] = fx::dissipation2(x, im, c->obj_weight, p.md.cv_diss);
     for (int k = 0; k < 9; ++k) src[9 * i + k] = src64[9 * i + k] = 0.;
-    dim[i] = fx::dissipation2_source(x, im, 1., p.fix.cv, src + 9 * i);
+    const fx::Dissipation2 d(x, fx::Factor(im), p.fix.cv);
+    dim[i] = d.dim;
+    // in the units of an adjoint of size 2^e (e from -40 to 20 over the cells)
+    // where it fits there, else in FP64
+    fx::Block b;
+    const double size[1] = {ldexp(1.3, i % 61 - 40)};
+    b.measure<1>(size);
+    const fx::Source2 r = d.scaled(p.fix, b);
+    if (r.on) {
+      *scaled += 1;
+      src[9 * i] = b.store(r.ev[0]);
+      static_for<4>([&](auto D) {
+        constexpr int k = decltype(D)::value + 1;
+        const fx::i64 eg = e_dot<LAT_D2Q9, k>(r.gx, r.gy, (fx::i64)0);
+        src[9 * i + k] = b.store(r.ev[k] + eg);
+        src[9 * i + k + 4] = b.store(r.ev[k] - eg);
+      });
+    } else {
+      d.add(c->obj_weight, src + 9 * i);
+    }
     val64[i] = ObjDissipation::evaluate<LAT_D2Q9, false>(f + 9 * i, g[i], 0, 0, 0, p);
     double dg = 0.;
     ObjDissipation::source<LAT_D2Q9, false>(f + 9 * i, g[i], src64 + 9 * i, dg, 0, 0, 0, p);

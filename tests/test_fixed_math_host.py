@@ -42,7 +42,7 @@ def lib():
     lib.fixed_forward.argtypes = [C.POINTER(G.CConfig), C.c_int, dp, dp, dp, dp]
     lib.fixed_reverse.argtypes = [C.POINTER(G.CConfig), C.c_int, dp, dp, dp, dp, dp, dp, dp]
     lib.fixed_thermal.argtypes = [C.c_int] + [dp] * 9
-    lib.fixed_dissipation.argtypes = [C.POINTER(G.CConfig), C.c_int] + [dp] * 7
+    lib.fixed_dissipation.argtypes = [C.POINTER(G.CConfig), C.c_int] + [dp] * 7 + [C.POINTER(C.c_int)]
     return lib
 
 
@@ -385,16 +385,21 @@ def test_fixed_thermal_is_at_least_as_exact_as_fp64(lib, spread):
         assert (np.abs(misc[:, k] - v)[keep] <= 2.0 ** -53 * np.abs(v)[keep] + 8 * 2.0 ** -58 * sl[keep, 0]).all()
 
 
+@pytest.mark.parametrize("weight", [1.0, 5e-4, -3.0])
 @pytest.mark.parametrize("amp", [1e-5, 0.01, 0.08])
-def test_fixed_dissipation_is_at_least_as_exact_as_fp64(lib, amp):
-    cfg = model("d2q9_bgk")
-    n = 4000
+def test_fixed_dissipation_is_at_least_as_exact_as_fp64(lib, amp, weight):
+    """Value, source (added to adjoints of sizes from 2^-40 to 2^20, whose units
+    take it or do not) and derivative by imult."""
+    cfg = model("d2q9_bgk").replace(obj_weight=weight)
+    n = 6100
     f, g = states(cfg, n, 41, amp)
     c = cfg.to_c()
     val, val64, dim = np.zeros(n), np.zeros(n), np.zeros(n)
     src, src64 = np.zeros((n, 9)), np.zeros((n, 9))
+    scaled = C.c_int()
     assert lib.fixed_dissipation(C.byref(c), n, ptr(f), ptr(g), ptr(val), ptr(src), ptr(dim),
-                                 ptr(val64), ptr(src64)) == n
+                                 ptr(val64), ptr(src64), C.byref(scaled)) == n
+    assert n // 4 < scaled.value < n
     F, im, om = f.astype(LD), imult_of(cfg, g), LD(cfg.omega)
     E = E2[:, :2].astype(LD)
     j, rho = F @ E, F.sum(1)
@@ -406,9 +411,19 @@ def test_fixed_dissipation_is_at_least_as_exact_as_fp64(lib, amp):
     pe = np.einsum("qa,qb,nab->nq", E, E, V)
     pj = np.einsum("nab,nb->na", V, j)
     sref = 4 * im[:, None] * (j @ E.T) + 2 * cv * ((pe - tr[:, None] / 3) - 2 * (pj @ E.T))
-    ea, eb = relative(val, ref, LD(1)), relative(val64, ref, LD(1))
-    sa, sb = relative(src, sref, LD(1)), relative(src64, sref, LD(1))
+    w = LD(weight)
+    # the source's error where the adjoint it joins is no larger than the weight
+    # (else it is the adjoint's own rounding that counts)
+    small = (np.arange(n) % 61 - 40) <= np.log2(abs(weight))
+    ea, eb = relative(val, w * ref, w), relative(val64, w * ref, w)
+    sa, sb = relative(src[small], (w * sref)[small], w), relative(src64[small], (w * sref)[small], w)
     print("dissipation", amp, "value: fixed", ea, "fp64", eb, "source: fixed", sa, "fp64", sb)
     assert ea <= 1.05 * eb and sa <= 1.05 * sb
+    size = 1.3 * 2.0 ** (np.arange(n) % 61 - 40)
+    # a diagonal population adds two components of g (four-fold products of
+    # V j, each of four products) and an even part: below 32 units in all
+    assert (np.abs(src - w * sref).astype(float) <=
+            (32 * 2.0 ** -61 * abs(weight) + 8 * 2.0 ** -57 * size)[:, None] +
+            2.0 ** -53 * np.abs(w * sref).astype(float)).all()
     # three roundings of 2 j^2 <= 4 (1.2 amp)^2, and j itself within 2^-61
     assert np.abs(dim - 2 * (j * j).sum(1)).max() < 3 * 2.0 ** -53 * 6 * amp * amp + 2.0 ** -58 * amp
