@@ -177,6 +177,11 @@ struct lbm_handle {
   unsigned* counter = nullptr;
   double* jdev = nullptr;
   size_t jcap = 0;
+  double* jhost = nullptr;       // one result in mapped host memory, and its device address
+  double* jhost_dev = nullptr;
+  double* step_partial = nullptr;   // warp partials of kept steps (lbm_forward's J_steps)
+  int step_rows = 0;                // steps it holds
+  double* step_row = nullptr;       // the row the next objective adds into (null: `partial`)
   double* stage = nullptr;     // FP64 AoS staging (ncell*Q)
   double* init_mac = nullptr;  // initial macros kept for lbm_gradient (device, may be null)
   std::vector<void*> slots;
@@ -222,11 +227,14 @@ int fail(lbm_handle* h, int code, const char* fmt, ...) {
     if (e_ != cudaSuccess) return fail((h), LBM_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
   } while (0)
 
-// *out = sum of partial[0..n) in a fixed order (one block of 1024 threads):
-// the objective summed over time steps by the accumulating reductions.
+// out[b] = sum of row b of partial (n values) in a fixed order, one block of
+// 1024 threads a row: the objective added up by the accumulating reductions,
+// over the time steps of a sweep (one row) or of single steps (a row each).
 __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict__ partial,
                                                        long long n, double* __restrict__ out) {
   __shared__ double sh[32];
+  partial += blockIdx.x * n;
+  out += blockIdx.x;
   double acc = 0.;
   for (long long i = threadIdx.x; i < n; i += blockDim.x) acc += partial[i];
 #pragma unroll
@@ -413,7 +421,7 @@ void destroy_buffers(lbm_handle* h) {
     if (s) cudaFree(s);
   h->slots.clear();
   void* ps[] = {h->gamma,  h->im,      h->dimult,  h->om6,  h->domega, h->sens,
-                h->partial, h->counter, h->jdev, h->stage, h->init_mac};
+                h->partial, h->counter, h->jdev, h->stage, h->init_mac, h->step_partial};
   for (void* p : ps)
     if (p) cudaFree(p);
   for (int k = 0; k < LBM_MAX_BC; ++k) {
@@ -427,7 +435,9 @@ void destroy_buffers(lbm_handle* h) {
   h->dimult = h->domega = nullptr;
   h->om6 = nullptr;
   h->counter = nullptr;
-  h->jdev = h->stage = h->init_mac = nullptr;
+  h->jdev = h->stage = h->init_mac = h->step_partial = nullptr;
+  if (h->jhost) cudaFreeHost(h->jhost);
+  h->jhost = h->jhost_dev = nullptr;
   for (cudaEvent_t& e : h->ev)
     if (e) {
       cudaEventDestroy(e);
@@ -512,7 +522,7 @@ KParams base_params(const lbm_handle* h, int t) {
   mf.cv_diss = (float)md.cv_diss;
   mf.obj_p[0] = (float)md.obj_p[0];
   mf.obj_p[1] = (float)md.obj_p[1];
-  p.partial = h->partial;
+  p.partial = h->step_row ? h->step_row : h->partial;
   p.counter = h->counter;
   p.accumulate = h->accumulate ? 1 : 0;
   p.gamma = h->gamma;
@@ -558,6 +568,26 @@ int ensure_jcap(lbm_handle* h, size_t n) {
   size_t cap = n < 1024 ? 1024 : n;
   CUDA_OR_FAIL(h, cudaMalloc(&h->jdev, cap * sizeof(double)));
   h->jcap = cap;
+  return 0;
+}
+
+int ensure_jhost(lbm_handle* h) {
+  if (h->jhost) return 0;
+  double* v = nullptr;
+  CUDA_OR_FAIL(h, cudaHostAlloc((void**)&v, sizeof(double), cudaHostAllocMapped));
+  h->jhost = v;
+  CUDA_OR_FAIL(h, cudaHostGetDevicePointer((void**)&h->jhost_dev, v, 0));
+  return 0;
+}
+
+// Rows for the objectives of up to 64 single steps, within 32 MB.
+int ensure_step_rows(lbm_handle* h) {
+  if (h->step_partial) return 0;
+  const size_t row = h->partial_cap * sizeof(double);
+  size_t rows = ((size_t)32 << 20) / row;
+  rows = rows < 1 ? 1 : rows > 64 ? 64 : rows;
+  CUDA_OR_FAIL(h, cudaMalloc(&h->step_partial, rows * row));
+  h->step_rows = (int)rows;
   return 0;
 }
 
@@ -1043,6 +1073,72 @@ int lbm_forward_steady(lbm_handle* h, int max_steps, int check_every, double tol
   return LBM_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// Blocks up to which one state's objective is reduced by the objective kernel
+// itself (its last block adds the blocks' sums, which queue for one counter)
+// instead of through the warp partials, their zeroing and a summing kernel:
+// one step of a 64x48 channel with its objective took 40 us that way, 26 so.
+constexpr unsigned kDirectBlocks = 2048;
+
+// lbm_forward with the objective of every step: each step adds into a row of
+// warp partials of its own, and one kernel sums the rows of up to 64 steps.
+// (A reduction to one value in every step, through a counter that all blocks
+// queue for, cost the 250x121x115 FP16 duct 128 us a step against 85 without.)
+int forward_per_step(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
+  int rc = ensure_jcap(h, (size_t)nsteps);
+  if (!rc) rc = ensure_step_rows(h);
+  if (rc) return rc;
+  const size_t cap = h->partial_cap;
+  int row = 0, done = 0;   // rows in use, values summed
+  // the next objective's row; before the first one, after the rows are summed
+  auto next_row = [&]() -> int {
+    if (row == 0) {
+      const int n = std::min(h->step_rows, nsteps - done);
+      CUDA_OR_FAIL(h, cudaMemsetAsync(h->step_partial, 0, n * cap * sizeof(double), h->stream));
+    }
+    h->step_row = h->step_partial + (size_t)row * cap;
+    ++row;
+    return 0;
+  };
+  auto sum_rows = [&](bool last) -> int {
+    if (row < h->step_rows && !last) return 0;
+    k_sum_partials<<<row, 1024, 0, h->stream>>>(h->step_partial, (long long)cap, h->jdev + done);
+    h->launches++;
+    CUDA_OR_FAIL(h, cudaGetLastError());
+    done += row;
+    row = 0;
+    return 0;
+  };
+  h->accumulate = true;
+  for (int k = 0; k < nsteps && !rc; ++k) {
+    // step k evaluates the state that step k-1 made
+    if (k > 0 && (rc = next_row())) break;
+    if ((rc = forward_step(h, k > 0 ? h->jdev : nullptr))) break;
+    if (k > 0) rc = sum_rows(false);
+  }
+  if (!rc) rc = next_row();
+  if (!rc) rc = objective_only(h, h->jdev);
+  if (!rc) rc = sum_rows(true);
+  h->accumulate = false;
+  h->step_row = nullptr;
+  if (rc || (rc = sync(h))) return rc;
+  std::vector<double> js((size_t)nsteps);
+  CUDA_OR_FAIL(h, cudaMemcpy(js.data(), h->jdev, js.size() * sizeof(double), cudaMemcpyDeviceToHost));
+  double acc = 0.;
+  for (int k = 0; k < nsteps; ++k) acc += js[k];
+  if (!std::isfinite(acc)) return fail(h, LBM_ERR_NONFINITE, "objective is not finite");
+  memcpy(J_steps, js.data(), js.size() * sizeof(double));
+  if (J_sum) *J_sum = acc;
+  return LBM_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 int lbm_forward(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
   if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
   if (nsteps < 0) return fail(h, LBM_ERR_ARG, "nsteps %d < 0", nsteps);
@@ -1050,42 +1146,33 @@ int lbm_forward(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
   if (!h->have_state) return fail(h, LBM_ERR_STATE, "no state (lbm_init_equilibrium)");
   if (J_sum) *J_sum = 0.;
   if (nsteps == 0) return LBM_OK;
-  bool obj = h->cfg.objective != LBM_OBJ_NONE;
-  int rc = ensure_jcap(h, (size_t)nsteps);
-  if (rc) return rc;
-  const bool sum_only = obj && !J_steps;
-  if (sum_only && (rc = begin_accumulate(h))) return rc;
-  for (int k = 0; k < nsteps; ++k) {
-    rc = forward_step(h, (obj && k > 0) ? h->jdev + (k - 1) : nullptr);
-    if (rc) {
-      h->accumulate = false;
-      return rc;
-    }
+  const bool obj = h->cfg.objective != LBM_OBJ_NONE;
+  int rc;
+  if (!obj) {
+    for (int k = 0; k < nsteps; ++k)
+      if ((rc = forward_step(h, nullptr))) return rc;
+    if ((rc = sync(h))) return rc;
+    if (J_steps) memset(J_steps, 0, sizeof(double) * nsteps);
+    return LBM_OK;
   }
-  if (obj) {
-    rc = objective_only(h, h->jdev + (nsteps - 1));
-    if (!rc && sum_only) rc = end_accumulate(h, h->jdev);
+  if (J_steps) return forward_per_step(h, nsteps, J_steps, J_sum);
+  if ((rc = ensure_jhost(h))) return rc;
+  if (nsteps == 1 && h->geo.nblocks <= kDirectBlocks) {
+    // one state's objective: the objective kernel reduces it by itself
+    if ((rc = forward_step(h, nullptr))) return rc;
+    if ((rc = objective_only(h, h->jhost_dev))) return rc;
+  } else {
+    if ((rc = begin_accumulate(h))) return rc;
+    for (int k = 0; k < nsteps && !rc; ++k) rc = forward_step(h, k > 0 ? h->jhost_dev : nullptr);
+    if (!rc) rc = objective_only(h, h->jhost_dev);
+    if (!rc) rc = end_accumulate(h, h->jhost_dev);
     h->accumulate = false;
     if (rc) return rc;
   }
-  rc = sync(h);
-  if (rc) return rc;
-  if (sum_only) {
-    double acc = 0.;
-    CUDA_OR_FAIL(h, cudaMemcpy(&acc, h->jdev, sizeof(double), cudaMemcpyDeviceToHost));
-    if (!std::isfinite(acc)) return fail(h, LBM_ERR_NONFINITE, "objective is not finite");
-    if (J_sum) *J_sum = acc;
-  } else if (obj) {
-    std::vector<double> js((size_t)nsteps);
-    CUDA_OR_FAIL(h, cudaMemcpy(js.data(), h->jdev, js.size() * sizeof(double), cudaMemcpyDeviceToHost));
-    double acc = 0.;
-    for (int k = 0; k < nsteps; ++k) acc += js[k];
-    if (!std::isfinite(acc)) return fail(h, LBM_ERR_NONFINITE, "objective is not finite");
-    if (J_steps) memcpy(J_steps, js.data(), js.size() * sizeof(double));
-    if (J_sum) *J_sum = acc;
-  } else if (J_steps) {
-    memset(J_steps, 0, sizeof(double) * nsteps);
-  }
+  if ((rc = sync(h))) return rc;
+  const double acc = *h->jhost;
+  if (!std::isfinite(acc)) return fail(h, LBM_ERR_NONFINITE, "objective is not finite");
+  if (J_sum) *J_sum = acc;
   return LBM_OK;
 }
 
@@ -2141,25 +2228,28 @@ int lbm_batch_forward(lbm_batch* b, int nsteps, double* J) {
   for (int i = 0; i < b->n; ++i) {
     if (!b->h[i]->have_design || !b->h[i]->have_state)
       return bfail(b, LBM_ERR_STATE, "lattice %d has no design or state", i);
-    if (ensure_jcap(b->h[i], (size_t)nsteps)) return bfail(b, LBM_ERR_MEM, "%s", b->h[i]->err.c_str());
+    if (ensure_jcap(b->h[i], 1)) return bfail(b, LBM_ERR_MEM, "%s", b->h[i]->err.c_str());
   }
-  int rc;
+  // objectives summed in the warp partials, as a gradient's forward sweep does
+  int rc = 0;
   double* res[LBM_MAX_BATCH];
-  for (int s = 0; s < nsteps; ++s) {
-    for (int i = 0; i < b->n; ++i) res[i] = s >= 1 ? b->h[i]->jdev + (s - 1) : nullptr;
-    if ((rc = batch_forward(b, res))) return rc;
-  }
-  for (int i = 0; i < b->n; ++i) res[i] = b->h[i]->jdev + (nsteps - 1);
-  if ((rc = batch_objective(b, kCurState, res))) return rc;
+  for (int i = 0; i < b->n; ++i) res[i] = b->h[i]->jdev;
+  for (int i = 0; i < b->n && !rc; ++i)
+    if (b->h[i]->cfg.objective != LBM_OBJ_NONE && (rc = begin_accumulate(b->h[i], b->stream)))
+      bfail(b, rc, "%s", b->h[i]->err.c_str());
+  for (int s = 0; s < nsteps && !rc; ++s) rc = batch_forward(b, s >= 1 ? res : nullptr);
+  if (!rc) rc = batch_objective(b, kCurState, res);
+  for (int i = 0; i < b->n && !rc; ++i)
+    if (b->h[i]->cfg.objective != LBM_OBJ_NONE &&
+        (rc = end_accumulate(b->h[i], b->h[i]->jdev, b->stream)))
+      bfail(b, rc, "%s", b->h[i]->err.c_str());
+  for (int i = 0; i < b->n; ++i) b->h[i]->accumulate = false;
+  if (rc) return rc;
   BCUDA(b, cudaStreamSynchronize(b->stream));
-  if (J) {
-    std::vector<double> js((size_t)nsteps);
-    for (int i = 0; i < b->n; ++i) {
-      BCUDA(b, cudaMemcpy(js.data(), b->h[i]->jdev, js.size() * sizeof(double), cudaMemcpyDeviceToHost));
-      double acc = 0.;
-      for (double v : js) acc += v;
-      J[i] = acc;
-    }
+  for (int i = 0; J && i < b->n; ++i) {
+    J[i] = 0.;
+    if (b->h[i]->cfg.objective != LBM_OBJ_NONE)
+      BCUDA(b, cudaMemcpy(&J[i], b->h[i]->jdev, sizeof(double), cudaMemcpyDeviceToHost));
   }
   return LBM_OK;
 }
