@@ -17,6 +17,7 @@
 
 #include "../../include/lbmgpu.h"
 #include "fixed_model.hpp"
+#include "host_buffers.hpp"
 #include "lbm_device.cuh"
 #include "lbm_ops.h"
 #include "state_pool.hpp"
@@ -177,8 +178,8 @@ struct lbm_handle {
   unsigned* counter = nullptr;
   double* jdev = nullptr;
   size_t jcap = 0;
-  double* jhost = nullptr;       // one result in mapped host memory, and its device address
-  double* jhost_dev = nullptr;
+  double* jhost = nullptr;       // a result and a flag in mapped host memory, and their
+  double* jhost_dev = nullptr;   // device address
   double* step_partial = nullptr;   // warp partials of kept steps (lbm_forward's J_steps)
   int step_rows = 0;                // steps it holds
   double* step_row = nullptr;       // the row the next objective adds into (null: `partial`)
@@ -246,6 +247,13 @@ __global__ void __launch_bounds__(1024) k_sum_partials(const double* __restrict_
     for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) tot += sh[w];
     *out = tot;
   }
+}
+
+// *bad = 1 if a value lies outside [0,1] or is not a number.
+__global__ void k_check_unit(const double* __restrict__ v, long long n, int* bad) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    if (!(v[i] >= 0. && v[i] <= 1.)) *bad = 1;
 }
 
 // sens[c] += coef * (*J) over the cells of box b (x fastest): the design
@@ -571,10 +579,13 @@ int ensure_jcap(lbm_handle* h, size_t n) {
   return 0;
 }
 
+// Design values from which on the range check runs on the device.
+constexpr int64_t kDeviceCheck = 8192;
+
 int ensure_jhost(lbm_handle* h) {
   if (h->jhost) return 0;
   double* v = nullptr;
-  CUDA_OR_FAIL(h, cudaHostAlloc((void**)&v, sizeof(double), cudaHostAllocMapped));
+  CUDA_OR_FAIL(h, cudaHostAlloc((void**)&v, 2 * sizeof(double), cudaHostAllocMapped));
   h->jhost = v;
   CUDA_OR_FAIL(h, cudaHostGetDevicePointer((void**)&h->jhost_dev, v, 0));
   return 0;
@@ -980,16 +991,35 @@ int lbm_set_bc_profile(lbm_handle* h, int k, int nt, int ncomp, const double* ta
 int lbm_set_design(lbm_handle* h, const double* gamma) {
   if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
   if (!gamma) return fail(h, LBM_ERR_ARG, "null design pointer");
-  for (int64_t i = 0; i < h->ncell; ++i) {
-    double g = gamma[i];
-    if (!std::isfinite(g)) return fail(h, LBM_ERR_NONFINITE, "design value %lld is not finite", (long long)i);
-    if (g < 0. || g > 1.) return fail(h, LBM_ERR_ARG, "design value %lld = %g outside [0,1]", (long long)i, g);
-  }
-  int rc = ensure_stage(h);
+  auto check = [&]() -> int {
+    for (int64_t i = 0; i < h->ncell; ++i) {
+      double g = gamma[i];
+      if (!std::isfinite(g)) return fail(h, LBM_ERR_NONFINITE, "design value %lld is not finite", (long long)i);
+      if (g < 0. || g > 1.) return fail(h, LBM_ERR_ARG, "design value %lld = %g outside [0,1]", (long long)i, g);
+    }
+    return 0;
+  };
+  // Large designs are checked on the device, before they replace the old one
+  // (the loop above takes 1 ns a value: 4.2 ms for 256x128x128 against 0.3 ms
+  // for the upload and both kernels; a second launch and wait cost 8 us, which
+  // 8192 values take here); the loop then names the value.
+  const bool on_device = h->ncell >= kDeviceCheck;
+  int rc = on_device ? 0 : check();
   if (rc) return rc;
-  set_regen_denominator(h, gamma);
+  if ((rc = ensure_stage(h))) return rc;
   CUDA_OR_FAIL(h, cudaMemcpyAsync(h->stage, gamma, (size_t)h->ncell * sizeof(double),
                                   cudaMemcpyHostToDevice, h->stream));
+  if (on_device) {
+    if ((rc = ensure_jhost(h))) return rc;
+    volatile int* bad = (volatile int*)(h->jhost + 1);
+    *bad = 0;
+    k_check_unit<<<608, 256, 0, h->stream>>>(h->stage, (long long)h->ncell, (int*)(h->jhost_dev + 1));
+    h->launches++;
+    CUDA_OR_FAIL(h, cudaGetLastError());
+    if ((rc = sync(h))) return rc;
+    if (*bad && (rc = check())) return rc;
+  }
+  set_regen_denominator(h, gamma);
   KParams p = base_params(h, 0);
   rc = launch(h, K_GAMMA, p, h->stage);
   if (rc) return rc;
@@ -1193,6 +1223,7 @@ int lbm_get_populations(const lbm_handle* hc, double* f) {
   p.fin = h->f[h->cur];
   rc = launch(h, K_EXPORT, p, h->stage);
   if (rc) return rc;
+  populate(f, (size_t)h->ncell * h->Q * sizeof(double));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(f, h->stage, (size_t)h->ncell * h->Q * sizeof(double),
                                   cudaMemcpyDeviceToHost, h->stream));
   return sync(h);
@@ -1226,6 +1257,7 @@ int lbm_get_macros(const lbm_handle* hc, double* mac) {
   p.fin = h->f[h->cur];
   rc = launch(h, K_MACROS, p, h->stage);
   if (rc) return rc;
+  populate(mac, (size_t)h->ncell * h->nmac * sizeof(double));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(mac, h->stage, (size_t)h->ncell * h->nmac * sizeof(double),
                                   cudaMemcpyDeviceToHost, h->stream));
   return sync(h);
@@ -1265,6 +1297,7 @@ int lbm_get_adjoint(const lbm_handle* hc, double* lam) {
   p.lam_in = h->lam[h->lcur];
   rc = launch(h, K_EXPORT_ADJ, p, h->stage);
   if (rc) return rc;
+  populate(lam, (size_t)h->ncell * h->Q * sizeof(double));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(lam, h->stage, (size_t)h->ncell * h->Q * sizeof(double),
                                   cudaMemcpyDeviceToHost, h->stream));
   return sync(h);
@@ -1274,6 +1307,7 @@ int lbm_get_sensitivity(const lbm_handle* hc, double* sens) {
   lbm_handle* h = const_cast<lbm_handle*>(hc);
   if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
   if (!sens) return fail(h, LBM_ERR_ARG, "null output");
+  populate(sens, (size_t)h->ncell * sizeof(double));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(sens, h->sens, (size_t)h->ncell * sizeof(double),
                                   cudaMemcpyDeviceToHost, h->stream));
   return sync(h);
@@ -1420,6 +1454,7 @@ int gradient_run(lbm_handle* h, int nsteps, int nsnap, int schedule, SteadyPhase
   // the objective's design term shared by the box cells, from J
   if (obj && (rc = add_design_term(h, h->jdev))) return rc;
   cudaEventRecord(h->ev[2], h->stream);
+  populate(dJdgamma, (size_t)h->ncell * sizeof(double));   // while the GPU works
   if ((rc = sync(h))) return rc;
   double acc = 0.;
   if (obj) {
@@ -2340,6 +2375,8 @@ int lbm_batch_gradient_schedule(lbm_batch* b, int nsteps, int nsnap, int schedul
     if ((rc = batch_sequence(b, nsteps, nsnap, schedule, &recomputed))) return rc;
   }
   cudaEventRecord(b->ev[1], b->stream);
+  for (int i = 0; dJdgamma && i < b->n; ++i)   // while the GPU works
+    populate(dJdgamma[i], (size_t)b->h[i]->ncell * sizeof(double));
   BCUDA(b, cudaStreamSynchronize(b->stream));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, b->ev[0], b->ev[1]);

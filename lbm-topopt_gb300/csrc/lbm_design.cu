@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "../../include/lbmgpu.h"
+#include "host_buffers.hpp"
 #include "lbm_ops.h"
 
 namespace {
@@ -309,6 +310,16 @@ __global__ void __launch_bounds__(kThreads) k_box_sum(Grid g, const int* __restr
     acc[0] += full[((long long)z * g.ny + y) * g.nx + x];
   }
   grid_reduce_values<1, false>(acc, red);
+}
+
+// 1 if a value lies outside [0,1] or is not a number, else 0
+__global__ void __launch_bounds__(kThreads) k_outside_unit(const double* __restrict__ v, long long n,
+                                                           Reduction red) {
+  double acc[1] = {0.};
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x)
+    if (!(v[i] >= 0. && v[i] <= 1.)) acc[0] = 1.;
+  grid_reduce_values<1, true>(acc, red);
 }
 
 __global__ void __launch_bounds__(kThreads) k_max_abs_diff(const double* __restrict__ a,
@@ -861,9 +872,15 @@ int lbm_topopt_num_variables(const lbm_topopt* t, int64_t* n) {
 
 int lbm_topopt_set_variables(lbm_topopt* t, const double* x) {
   if (!t || !x) return tfail(t, LBM_ERR_ARG, "null argument");
-  for (long long i = 0; i < t->n; ++i)
+  // checked on the device before they replace the old ones; the loop names the value
+  TCUDA(t, cudaMemcpyAsync(t->tmp2, x, sizeof(double) * t->n, cudaMemcpyHostToDevice, t->st));
+  k_outside_unit<<<reduce_grid(t->n), kThreads, 0, t->st>>>(t->tmp2, t->n, reduction(t));
+  double outside = 0.;
+  int rc = reduced(t, 1, &outside);
+  if (rc) return rc;
+  for (long long i = 0; outside > 0. && i < t->n; ++i)
     if (!(x[i] >= 0. && x[i] <= 1.)) return tfail(t, LBM_ERR_ARG, "design variable %lld outside [0,1]", i);
-  TCUDA(t, cudaMemcpyAsync(t->x, x, sizeof(double) * t->n, cudaMemcpyHostToDevice, t->st));
+  TCUDA(t, cudaMemcpyAsync(t->x, t->tmp2, sizeof(double) * t->n, cudaMemcpyDeviceToDevice, t->st));
   TCUDA(t, cudaStreamSynchronize(t->st));
   for (int r = 0; r < t->nreal; ++r) t->have_sens[r] = false;
   return LBM_OK;
@@ -872,6 +889,7 @@ int lbm_topopt_set_variables(lbm_topopt* t, const double* x) {
 int lbm_topopt_get_variables(const lbm_topopt* t, double* x) {
   if (!t || !x) return tfail(nullptr, LBM_ERR_ARG, "null argument");
   lbm_topopt* tt = const_cast<lbm_topopt*>(t);
+  lbm::populate(x, sizeof(double) * t->n);
   TCUDA(tt, cudaMemcpyAsync(x, t->x, sizeof(double) * t->n, cudaMemcpyDeviceToHost, t->st));
   TCUDA(tt, cudaStreamSynchronize(t->st));
   return LBM_OK;
@@ -891,6 +909,7 @@ int lbm_topopt_physical(lbm_topopt* t, int r, double* gamma) {
   if (r < 0 || r >= t->nreal) return tfail(t, LBM_ERR_ARG, "no realisation %d", r);
   int rc = forward_chain(t, r);
   if (rc) return rc;
+  lbm::populate(gamma, sizeof(double) * t->g.n);   // while the GPU works
   TCUDA(t, cudaMemcpyAsync(gamma, t->gamma[r], sizeof(double) * t->g.n, cudaMemcpyDeviceToHost, t->st));
   TCUDA(t, cudaStreamSynchronize(t->st));
   return LBM_OK;
@@ -954,6 +973,7 @@ int lbm_topopt_get_design_sensitivity(const lbm_topopt* t, int r, double* dJdx) 
   lbm_topopt* tt = const_cast<lbm_topopt*>(t);
   if (r < 0 || r >= t->nreal) return tfail(tt, LBM_ERR_ARG, "no realisation %d", r);
   if (!t->have_sens[r]) return tfail(tt, LBM_ERR_STATE, "no sensitivity set for realisation %d", r);
+  lbm::populate(dJdx, sizeof(double) * t->n);
   TCUDA(tt, cudaMemcpyAsync(dJdx, t->df[r], sizeof(double) * t->n, cudaMemcpyDeviceToHost, t->st));
   TCUDA(tt, cudaStreamSynchronize(t->st));
   return LBM_OK;
