@@ -2,12 +2,19 @@
 // (lbm_fixed.cuh), computed on the host once per handle.
 #pragma once
 
+#include <climits>
 #include <cmath>
 
 #include "../../include/lbmgpu.h"
 #include "lbm_device.cuh"
+#include "lbm_ops.h"
 
 namespace lbm {
+
+inline bool velocity_objective(const lbm_config& c) {
+  return c.objective == LBM_OBJ_THROUGH_FLOW || c.objective == LBM_OBJ_OUTFLOW ||
+         c.objective == LBM_OBJ_HEAT_FLUX;
+}
 
 // v * 2^bits as an even unsigned constant; clears ok where it does not fit.
 inline unsigned long long fixed_constant(long double v, int bits, bool& ok) {
@@ -24,16 +31,10 @@ inline unsigned long long fixed_constant(long double v, int bits, bool& ok) {
 inline FixedModel fixed_model(const lbm_config& c) {
   FixedModel m = {};
   if (c.storage != LBM_STORE_FP64) return m;
-  // A velocity objective of a flow that is still at rest is nothing but
-  // rounding.  With one, cells at rest keep the FP64 expressions, whose
-  // rounding is the reference's, and so do all cells of lattices so small that
-  // it shows next to the objective of a moving flow (12 cells to average over
-  // on 36x36).  The cost is the start-up of the flow: 201x201 pump, 600 steps,
-  // 26 against 14 ms (71 ms in FP64); 36x36 MRT step 7.4 against 3.4 us.
-  m.rest = c.objective == LBM_OBJ_THROUGH_FLOW || c.objective == LBM_OBJ_OUTFLOW ||
-           c.objective == LBM_OBJ_HEAT_FLUX;
+  // lattices too small for a velocity objective to stand clear of rounding
+  // (12 cells to average over on 36x36, MRT step 7.4 against 3.4 us)
   const int64_t ncell = (int64_t)c.nx * c.ny * (c.lattice == LBM_D3Q19 ? c.nz : 1);
-  if (m.rest && ncell < 2048) return m;
+  if (velocity_objective(c) && ncell < 2048) return m;
   bool ok = true;
   const long double om = c.omega;
   if (c.lattice == LBM_D3Q19 && c.collision == LBM_MRT) {
@@ -73,6 +74,49 @@ inline FixedModel fixed_model(const lbm_config& c) {
   if (!weight) ok = ok && c.objective != LBM_OBJ_DISSIPATION;
   m.ok = ok ? 1 : 0;
   return m;
+}
+
+// A velocity objective of a flow that is still at rest is nothing but rounding:
+// sweeps too short for the flow to reach the objective's cells keep the FP64
+// operators, whose rounding is the reference's.
+//
+// Steps after which a velocity objective measures a flow and no longer the
+// rounding of one at rest: one and a half times what sound (1/sqrt(3) cells a
+// step) takes from the nearest boundary that drives the flow to the cells that
+// the objective averages over, and 100.  (A heat flux sums over its box, where
+// only the warm part counts: to the middle.)  On the 201x201 pump the
+// pressure wave takes 164 steps to the outlets; its objective is 3e-10 after
+// 150 steps and 1e-6 after 250.  INT_MAX where no boundary drives the flow.
+// 0 for the other objectives.
+inline int flow_start_up(const lbm_config& c) {
+  ObjectiveInfo oi;
+  if (!velocity_objective(c) || !objective_info(c.objective, &oi)) return 0;
+  double best = -1.;
+  for (int k = 0; k < c.nbc; ++k) {
+    const lbm_bc& b = c.bc[k];
+    const bool velocity = b.kind == LBM_BC_VELOCITY || b.kind == LBM_BC_VELOCITY_STANDARD;
+    const bool pressure = b.kind == LBM_BC_PRESSURE || b.kind == LBM_BC_PRESSURE_STANDARD;
+    const bool drives = (velocity && (b.value != 0. || b.profile == LBM_PROFILE_TABLE)) ||
+                        (pressure && (b.value != 1. || b.amp != 0. || b.profile == LBM_PROFILE_TABLE ||
+                                      b.time_law != LBM_TIME_OFFSET_SINE));
+    if (!drives) continue;
+    for (int side = 0; side < 2; ++side) {
+      if (!(oi.uses & (side ? kUsesOut : kUsesIn))) continue;
+      const int* o = side ? c.obj_out : c.obj_in;
+      double d2 = 0.;
+      for (int a = 0; a < 3; ++a) {
+        const int lo = o[2 * a] - b.box[2 * a + 1], hi = b.box[2 * a] - o[2 * a + 1];
+        double gap = lo > hi ? lo : hi;
+        if (c.objective == LBM_OBJ_HEAT_FLUX) {
+          const double mid = 0.5 * (o[2 * a] + o[2 * a + 1]);
+          gap = fmax(mid - b.box[2 * a + 1], b.box[2 * a] - mid);
+        }
+        if (gap > 0.) d2 += gap * gap;
+      }
+      if (best < 0. || d2 < best) best = d2;
+    }
+  }
+  return best < 0. ? INT_MAX : (int)(1.5 * sqrt(3. * best)) + 100;
 }
 
 }  // namespace lbm

@@ -169,6 +169,8 @@ struct lbm_handle {
   void* lam[2] = {nullptr, nullptr};
   int lcur = 0;
   FixedModel fix = {};                 // fixed-point form of the FP64 collision
+  int start_up = 0;                    // steps until the objective sees the flow (flow_start_up)
+  int horizon = 0;                     // last step of the sweep being taken
   unsigned long long* im = nullptr;    // its porosity planes (KParams::im, dimult)
   double* dimult = nullptr;
   unsigned long long* om6 = nullptr;   // and the thermal lattice's (om6, domega)
@@ -537,6 +539,7 @@ KParams base_params(const lbm_handle* h, int t) {
   p.sens = h->sens;
   p.sens_atomic = h->sens_atomic ? 1 : 0;
   p.fix = h->fix;
+  if (h->horizon < h->start_up) p.fix.ok = 0;
   p.im = h->im;
   p.dimult = h->dimult;
   p.om6 = h->om6;
@@ -567,6 +570,11 @@ int launch(lbm_handle* h, int kind, const KParams& p, double* aux) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(h, LBM_ERR_CUDA, "kernel launch %d: %s", kind, cudaGetErrorString(e));
   return 0;
+}
+
+// The step that n more steps lead to.
+int end_step(const lbm_handle* h, int64_t n) {
+  return (int)std::min<int64_t>((int64_t)h->t + n, INT_MAX - 1);
 }
 
 int ensure_jcap(lbm_handle* h, size_t n) {
@@ -667,7 +675,7 @@ int adjoint_at(lbm_handle* h, const void* f) {
   p.lam_in = h->lam[h->lcur];
   p.lam_out = h->lam[1 - h->lcur];
   p.eval_obj = (h->t >= h->obj_from && h->cfg.objective != LBM_OBJ_NONE) ? 1 : 0;
-  int rc = launch(h, h->adj_lean || h->adj_wide ? K_ADJOINT_LEAN : K_ADJOINT, p, nullptr);
+  int rc = launch(h, h->adj_lean || (h->adj_wide && p.fix.ok) ? K_ADJOINT_LEAN : K_ADJOINT, p, nullptr);
   if (rc) return rc;
   h->lcur ^= 1;
   return 0;
@@ -875,6 +883,7 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   ALLOC(h->lam[1], adjoint_bytes(h));
   ALLOC(h->gamma, (size_t)h->P * h->gam_bytes);
   h->fix = fixed_model(c);
+  h->start_up = flow_start_up(c);
   if (h->fix.ok) {
     ALLOC(h->im, (size_t)h->P * sizeof(unsigned long long));
     ALLOC(h->dimult, (size_t)h->P * sizeof(double));
@@ -1083,6 +1092,7 @@ int lbm_forward_steady(lbm_handle* h, int max_steps, int check_every, double tol
   if (!h->have_state) return fail(h, LBM_ERR_STATE, "no state (lbm_init_equilibrium)");
   int rc = ensure_jcap(h, 1);
   if (rc) return rc;
+  h->horizon = end_step(h, max_steps);
   unsigned long long* bits = (unsigned long long*)h->jdev;
   double last = -1.;
   int k = 0;
@@ -1178,6 +1188,7 @@ int lbm_forward(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
   if (nsteps == 0) return LBM_OK;
   const bool obj = h->cfg.objective != LBM_OBJ_NONE;
   int rc;
+  h->horizon = end_step(h, nsteps);
   if (!obj) {
     for (int k = 0; k < nsteps; ++k)
       if ((rc = forward_step(h, nullptr))) return rc;
@@ -1276,6 +1287,7 @@ int lbm_adjoint_step(lbm_handle* h) {
   if (!h->have_design || !h->have_state) return fail(h, LBM_ERR_STATE, "no design or state");
   if (!h->have_adjoint) return fail(h, LBM_ERR_STATE, "adjoint not reset (lbm_adjoint_reset)");
   int rc;
+  h->horizon = std::max(h->horizon, h->t);
   if (h->cfg.objective == LBM_OBJ_REGENERATOR_EFFICIENCY && h->t >= h->obj_from) {
     // this step's share of the 1/D design term needs the step's objective
     if ((rc = ensure_jcap(h, 1))) return rc;
@@ -1391,6 +1403,8 @@ int gradient_run(lbm_handle* h, int nsteps, int nsnap, int schedule, SteadyPhase
 
   h->t_phase = INT_MAX;   // a new run: ramps wait for the steady phase
   h->obj_from = 1;
+  h->t = 0;
+  h->horizon = end_step(h, sp ? (int64_t)sp->max_steps + nsteps : nsteps);
   cudaEventRecord(h->ev[0], h->stream);
   {
     const int out = pool.scratch();
@@ -1519,6 +1533,8 @@ int lbm_time_steps(lbm_handle* h, int which, int nsteps, float* ms) {
     h->have_adjoint = true;
   }
   int t_keep = h->t;
+  const int horizon_keep = h->horizon;
+  h->horizon = INT_MAX;   // as in a long sweep
   if (which == 1 && h->t < 1) h->t = 1;
   cudaEventRecord(h->ev[0], h->stream);
   for (int k = 0; k < nsteps; ++k) {
@@ -1530,8 +1546,10 @@ int lbm_time_steps(lbm_handle* h, int which, int nsteps, float* ms) {
       rc = forward_step(h, nullptr);
       if (!rc) rc = adjoint_step(h);
     }
-    if (rc) return rc;
+    if (rc) break;
   }
+  h->horizon = horizon_keep;
+  if (rc) return rc;
   cudaEventRecord(h->ev[1], h->stream);
   if ((rc = sync(h))) return rc;
   if (which == 1) h->t = t_keep;
@@ -1548,7 +1566,8 @@ int lbm_autotune(lbm_handle* h, int nsteps) {
   void* keep = nullptr;
   CUDA_OR_FAIL(h, cudaMalloc(&keep, state_bytes(h)));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(keep, h->f[h->cur], state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
-  const int t_keep = h->t, cur_keep = h->cur;
+  const int t_keep = h->t, cur_keep = h->cur, horizon_keep = h->horizon;
+  h->horizon = INT_MAX;   // as in a long sweep
   if (!h->have_adjoint) {
     if ((rc = zero_adjoint(h))) { cudaFree(keep); return rc; }
     h->have_adjoint = true;
@@ -1593,6 +1612,7 @@ int lbm_autotune(lbm_handle* h, int nsteps) {
   h->tuned = true;
   h->cur = cur_keep;
   h->t = t_keep;
+  h->horizon = horizon_keep;
   CUDA_OR_FAIL(h, cudaMemcpyAsync(h->f[h->cur], keep, state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
   rc = zero_adjoint(h);
   if (!rc) rc = sync(h);
@@ -1951,6 +1971,8 @@ int batch_sequence(lbm_batch* b, int nsteps, int nsnap, int schedule, int64_t* r
   for (int i = 0; i < b->n; ++i) {
     b->h[i]->cur = 0;
     b->h[i]->lcur = 0;
+    b->h[i]->t = 0;
+    b->h[i]->horizon = nsteps;
   }
   WangSchedule ws(nsnap);
   const bool planned = schedule == LBM_SCHEDULE_STATIC;
@@ -2137,6 +2159,7 @@ int lbm_batch_autotune(lbm_batch* b, int nsteps) {
     for (void* p : h->lam) BCUDA(b, cudaMemsetAsync(p, 0, adjoint_bytes(h), b->stream));
     h->have_adjoint = true;
     h->t = 1;
+    h->horizon = INT_MAX;   // as in a long sweep
   }
   // each kernel on its own: every shape for the forward step, then every
   // shape and both register variants for the reverse step
@@ -2268,7 +2291,10 @@ int lbm_batch_forward(lbm_batch* b, int nsteps, double* J) {
   // objectives summed in the warp partials, as a gradient's forward sweep does
   int rc = 0;
   double* res[LBM_MAX_BATCH];
-  for (int i = 0; i < b->n; ++i) res[i] = b->h[i]->jdev;
+  for (int i = 0; i < b->n; ++i) {
+    res[i] = b->h[i]->jdev;
+    b->h[i]->horizon = end_step(b->h[i], nsteps);
+  }
   for (int i = 0; i < b->n && !rc; ++i)
     if (b->h[i]->cfg.objective != LBM_OBJ_NONE && (rc = begin_accumulate(b->h[i], b->stream)))
       bfail(b, rc, "%s", b->h[i]->err.c_str());
@@ -2415,6 +2441,7 @@ int lbm_batch_time_steps(lbm_batch* b, int which, int nsteps, float* ms) {
       h->have_adjoint = true;
     }
     if (which >= 1 && h->t < 1) h->t = 1;
+    h->horizon = INT_MAX;   // as in a long sweep
   }
   cudaEventRecord(b->ev[0], b->stream);
   for (int k = 0; k < nsteps; ++k) {

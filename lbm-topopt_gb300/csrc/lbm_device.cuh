@@ -253,7 +253,6 @@ struct ModelParams {
 // what c[] holds for each operator), filled once per handle by the host.
 struct FixedModel {
   int ok;                            // the model has a fixed-point form with these constants
-  int rest;                          // cells at rest take the FP64 operators
   int we3;                           // the D3Q19 MRT weight we differs from 3
   int wej_neg, wxx_neg, we3_neg;     // signs of the three below: 0 or -1
   unsigned long long c[12];          // factors below 1, times 2^64

@@ -175,16 +175,6 @@ struct Window {
   }
 };
 
-// Whether the cell is at rest: every component of j below 2^-40, which rounding
-// alone stays under for some 10,000 steps.
-template <int LAT>
-__device__ __forceinline__ bool at_rest(const i64* x) {
-  constexpr i64 kRest = 1ll << (kScale - 40);
-  i64 rho, jx, jy, jz;
-  flow_macros<LAT>(x, rho, jx, jy, jz);
-  return (((u64)(jx + kRest) | (u64)(jy + kRest) | (u64)(jz + kRest)) >> (kScale - 39)) == 0u;
-}
-
 // ---------------------------------------------------------------------------
 // D3Q19 MRT + partial bounce-back in population-pair form (mrt3d_pair_collide
 // with the equilibrium folded into the rows and the rates into the back-map).

@@ -30,7 +30,7 @@ namespace lbm {
 // slower); the D3Q19 BGK adjoint in increment form needs more registers than
 // 64 and gets 3 blocks (85); the FP64 kernels are FP64-throughput-bound on
 // GB300 and keep all their registers.
-template <int LAT, int COLL, class S>
+template <int LAT, int COLL, class S, bool FIXED = false>
 struct Occupancy {
   static constexpr int fwd = (LAT == LAT_D2Q9) ? 6 : 5;
   static constexpr int adj = (LAT == LAT_D3Q19 && COLL == LBM_BGK) ? 3 : 4;
@@ -51,10 +51,16 @@ struct Occupancy {
 // ones (wide_reverse in lbm_capi.cu): 4096x2048 0.332 -> 0.294 ms, 1024x512 with
 // dissipation 43.9 -> 41.1 us, but 128x64 6.2 -> 6.7 us and 201x201 7.8 -> 8.4 us.
 template <int LAT, int COLL>
-struct Occupancy<LAT, COLL, double> {
+struct Occupancy<LAT, COLL, double, true> {
   static constexpr int fwd = LAT == LAT_D2Q9 ? 3 : 2, adj = 2;
   static constexpr int adj_lean = LAT == LAT_D2Q9 ? 3 : 2, adj_lean_batch = adj_lean;
   static constexpr bool has_lean = LAT == LAT_D2Q9;
+};
+// the FP64 operators are bound by the FP64 pipe and keep all their registers
+template <int LAT, int COLL>
+struct Occupancy<LAT, COLL, double, false> {
+  static constexpr int fwd = 1, adj = 1, adj_lean = 1, adj_lean_batch = 1;
+  static constexpr bool has_lean = false;
 };
 
 template <class S>
@@ -308,7 +314,10 @@ static __device__ __noinline__ void add_dissipation_fp64(const fx::i64* x, unsig
   fx::Dissipation2(x, fx::Factor(im), p.fix.cv).add(p.md.obj_weight, lam);
 }
 
-// Whether the collision runs in fixed point: FP64 storage.
+// Whether the collision can run in fixed point: FP64 storage.  The step kernels
+// are built twice for it: FIXED ones, in which cells (and, in a batch, whole
+// lattices) may still take the FP64 operators, and FP64 ones without the
+// registers' bounds for launches that have no fixed-point cell.
 template <class S>
 constexpr bool kFixed = std::is_same<S, double>::value;
 
@@ -321,7 +330,9 @@ __device__ __forceinline__ bool fixed_porosity(unsigned long long im) {
 template <int LAT>
 struct FixedDesign {
   unsigned long long im, om6 = 0ull;
-  __device__ __forceinline__ FixedDesign(const KParams& p, int c) : im(p.im[c]) {
+  __device__ __forceinline__ FixedDesign(const KParams& p, int c) : im(~0ull) {
+    if (!p.fix.ok) return;
+    im = p.im[c];
     if constexpr (LAT == LAT_D2Q9_D2Q5) om6 = p.om6[c];
   }
   __device__ __forceinline__ bool ok() const { return fixed_porosity(im) && om6 != ~0ull; }
@@ -347,7 +358,6 @@ __device__ __forceinline__ double forward_cell_fixed(const KParams& p, int x, in
     xi[q] = w.template load<LAT, q>(f[q]);
   });
   bool ok = w.template ok<LAT>(xi) && des.ok();
-  if (p.fix.rest) ok = ok && !fx::at_rest<LAT>(xi);
   fx::ThermalBlock bt;
   if constexpr (THERMAL) {
     bt.template measure<5>(f + 9);
@@ -389,7 +399,7 @@ __device__ __forceinline__ double forward_cell_fixed(const KParams& p, int x, in
 
 // Forward step of cell (x,y,z); returns its objective contribution F(f_t).
 // in: warp_interior of the calling warp, read with WARP.
-template <int LAT, int COLL, class S, bool WARP>
+template <int LAT, int COLL, class S, bool WARP, bool FIXED>
 __device__ __forceinline__ typename Store<S>::C forward_cell(const KParams& p, int x, int y, int z,
                                                              bool in) {
   using L = Lattice<LAT>;
@@ -400,10 +410,8 @@ __device__ __forceinline__ typename Store<S>::C forward_cell(const KParams& p, i
     const int c = (z * p.ny + y) * p.nx + x;
     C f[L::Q];
     load_state<LAT, S>(f, (const S*)p.fin, c, (int)p.P);
-    if constexpr (kFixed<S>) {
-      if (p.fix.ok)
-        return forward_cell_fixed<LAT, COLL, WARP>(p, x, y, z, c, f, FixedDesign<LAT>(p, c), in);
-    }
+    if constexpr (FIXED)
+      return forward_cell_fixed<LAT, COLL, WARP>(p, x, y, z, c, f, FixedDesign<LAT>(p, c), in);
     objv = forward_cell_from<LAT, COLL, S, WARP>(p, x, y, z, c, f, C(((const G*)p.gamma)[c]), in);
   }
   return objv;
@@ -474,7 +482,7 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
                                 take_interior<LAT, WARP>(in, x, y, z, p), p);
   load_state<LAT, double>(f, (const double*)p.fin, c, (int)p.P);
   const FixedDesign<LAT> des(p, c);
-  const double dimult = p.dimult[c];
+  const double dimult = p.fix.ok ? p.dimult[c] : 0.;
   if (on_bc_face<LAT>(x, y, p)) apply_bcs<LAT, false>(f, x, y, z, p);
   double dg = 0.;
   fx::Block b;
@@ -487,7 +495,8 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
     zero = zero && l.zero;
     ok = ok && (l.zero || l.ok) && (g.zero || g.ok);
   }
-  const bool diss = L::DIM == 2 && p.eval_obj && p.objective == LBM_OBJ_DISSIPATION;
+  const bool diss =
+      L::DIM == 2 && p.fix.ok && p.eval_obj && p.objective == LBM_OBJ_DISSIPATION;
   // cells that no adjoint has reached yet keep their zeros
   if (!zero || diss) {
     fx::Window w;
@@ -497,8 +506,7 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
       xi[q] = w.template load<LAT, q>(f[q]);
     });
     ok = ok && w.template ok<LAT>(xi) && des.ok();
-    if (p.fix.rest) ok = ok && !fx::at_rest<LAT>(xi);
-    if (ok) {
+      if (ok) {
       const fx::Factor im(des.im);
       fx::Source2 src;
       double ddiss = 0.;
@@ -554,7 +562,7 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
 
 // Reverse step of cell (x,y,z); in: warp_interior of the calling warp, read
 // with WARP.
-template <int LAT, int COLL, class S, bool WARP>
+template <int LAT, int COLL, class S, bool WARP, bool FIXED>
 __device__ __forceinline__ void adjoint_cell(const KParams& p, int x, int y, int z, bool in) {
   using L = Lattice<LAT>;
   using C = typename Store<S>::C;
@@ -563,11 +571,9 @@ __device__ __forceinline__ void adjoint_cell(const KParams& p, int x, int y, int
   constexpr bool SHIFT = Store<S>::SHIFT;
   if (x >= p.nx || y >= p.ny) return;
   const int c = (z * p.ny + y) * p.nx + x;
-  if constexpr (kFixed<S>) {
-    if (p.fix.ok) {
-      adjoint_cell_fixed<LAT, COLL, WARP>(p, x, y, z, c, in);
-      return;
-    }
+  if constexpr (FIXED) {
+    adjoint_cell_fixed<LAT, COLL, WARP>(p, x, y, z, c, in);
+    return;
   }
   const A* __restrict__ lin = (const A*)p.lam_in;
   A* __restrict__ lout = (A*)p.lam_out;
@@ -678,26 +684,27 @@ __device__ __forceinline__ void step_prologue() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-template <int LAT, int COLL, class S>
-__global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S>::fwd) k_forward(KParams p) {
+template <int LAT, int COLL, class S, bool FIXED = false>
+__global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S, FIXED>::fwd) k_forward(KParams p) {
   step_prologue();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   constexpr bool W = kWarpInterior<LAT>;
   const bool in = W ? warp_interior<LAT>(x, y, blockIdx.z, p) : false;
-  const auto objv = forward_cell<LAT, COLL, S, W>(p, x, y, blockIdx.z, in);
+  const auto objv = forward_cell<LAT, COLL, S, W, FIXED>(p, x, y, blockIdx.z, in);
   if (p.eval_obj) grid_reduce(objv, p);
 }
 
-template <int LAT, int COLL, class S, bool LEAN = false>
-__global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S>::adj_lean
-                                            : Occupancy<LAT, COLL, S>::adj) k_adjoint(KParams p) {
+template <int LAT, int COLL, class S, bool LEAN = false, bool FIXED = false>
+__global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S, FIXED>::adj_lean
+                                            : Occupancy<LAT, COLL, S, FIXED>::adj)
+    k_adjoint(KParams p) {
   step_prologue();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   constexpr bool W = kWarpInterior<LAT>;
   const bool in = W ? warp_interior<LAT>(x, y, blockIdx.z, p) : false;
-  adjoint_cell<LAT, COLL, S, W>(p, x, y, blockIdx.z, in);
+  adjoint_cell<LAT, COLL, S, W, FIXED>(p, x, y, blockIdx.z, in);
 }
 
 // Objective of the state f_t alone (the last step of a forward sweep).
@@ -725,8 +732,8 @@ __device__ __forceinline__ int batch_lattice_of(const BatchParams& bp, int vb) {
   return i;
 }
 
-template <int LAT, int COLL, class S>
-__global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S>::fwd)
+template <int LAT, int COLL, class S, bool FIXED = false>
+__global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S, FIXED>::fwd)
     k_forward_batch(const __grid_constant__ BatchParams bp) {
   step_prologue();
   for (int vb = blockIdx.x; vb < bp.start[kMaxBatch]; vb += gridDim.x) {
@@ -744,16 +751,16 @@ __global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S>::fwd)
     double objv = 0.;
 #pragma unroll 1
     for (int k = 0; k < kBatchRowsForward; ++k) {
-      const auto v = forward_cell<LAT, COLL, S, false>(p, x, y + k * (int)blockDim.y, bz, false);
+      const auto v = forward_cell<LAT, COLL, S, false, FIXED>(p, x, y + k * (int)blockDim.y, bz, false);
       if (p.eval_obj) objv += (double)v;
     }
     if (p.eval_obj) grid_reduce_v(objv, p, lb, bp.start[i + 1] - bp.start[i]);
   }
 }
 
-template <int LAT, int COLL, class S, bool LEAN = false>
-__global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S>::adj_lean_batch
-                                            : Occupancy<LAT, COLL, S>::adj)
+template <int LAT, int COLL, class S, bool LEAN = false, bool FIXED = false>
+__global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S, FIXED>::adj_lean_batch
+                                            : Occupancy<LAT, COLL, S, FIXED>::adj)
     k_adjoint_batch(const __grid_constant__ BatchParams bp) {
   step_prologue();
   for (int vb = blockIdx.x; vb < bp.start[kMaxBatch]; vb += gridDim.x) {
@@ -766,7 +773,7 @@ __global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S>::adj_lean_
     const int y = (r - bz * bp.gy[i]) * (blockDim.y * kBatchRowsReverse) + threadIdx.y;
 #pragma unroll 1
     for (int k = 0; k < kBatchRowsReverse; ++k)
-      adjoint_cell<LAT, COLL, S, false>(p, x, y + k * (int)blockDim.y, bz, false);
+      adjoint_cell<LAT, COLL, S, false, FIXED>(p, x, y + k * (int)blockDim.y, bz, false);
   }
 }
 
@@ -985,17 +992,45 @@ void launch_overlapped(K kern, dim3 grid, dim3 block, cudaStream_t st, const P& 
 
 template <int LAT, int COLL, class S>
 struct OpsImpl {
+  // whether a lattice of the batch has fixed-point cells
+  static bool any_fixed(const BatchParams& bp) {
+    for (int i = 0; i < bp.n; ++i)
+      if (bp.p[i].fix.ok) return true;
+    return false;
+  }
+  template <bool FIXED>
+  static void launch_step(int kind, dim3 grid, dim3 block, cudaStream_t st, const KParams& p) {
+    using O = Occupancy<LAT, COLL, S, FIXED>;
+    if (kind == K_FORWARD)
+      launch_overlapped(k_forward<LAT, COLL, S, FIXED>, grid, block, st, p);
+    else if (kind == K_ADJOINT)
+      launch_overlapped(k_adjoint<LAT, COLL, S, false, FIXED>, grid, block, st, p);
+    else
+      launch_overlapped(k_adjoint<LAT, COLL, S, O::has_lean, FIXED>, grid, block, st, p);
+  }
+  template <bool FIXED>
+  static void launch_batch_step(int kind, dim3 grid, dim3 block, cudaStream_t st,
+                                const BatchParams& bp) {
+    using O = Occupancy<LAT, COLL, S, FIXED>;
+    if (kind == K_FORWARD)
+      launch_overlapped(k_forward_batch<LAT, COLL, S, FIXED>, grid, block, st, bp);
+    else if (kind == K_ADJOINT)
+      launch_overlapped(k_adjoint_batch<LAT, COLL, S, false, FIXED>, grid, block, st, bp);
+    else
+      launch_overlapped(k_adjoint_batch<LAT, COLL, S, O::has_lean, FIXED>, grid, block, st, bp);
+  }
   static void launch_batch(int kind, dim3 grid, dim3 block, cudaStream_t st, const BatchParams& bp) {
     switch (kind) {
       case K_FORWARD:
-        launch_overlapped(k_forward_batch<LAT, COLL, S>, grid, block, st, bp);
-        break;
       case K_ADJOINT:
-        launch_overlapped(k_adjoint_batch<LAT, COLL, S>, grid, block, st, bp);
-        break;
       case K_ADJOINT_LEAN:
-        launch_overlapped(k_adjoint_batch<LAT, COLL, S, Occupancy<LAT, COLL, S>::has_lean>, grid,
-                          block, st, bp);
+        if constexpr (kFixed<S>) {
+          if (any_fixed(bp)) {
+            launch_batch_step<true>(kind, grid, block, st, bp);
+            break;
+          }
+        }
+        launch_batch_step<false>(kind, grid, block, st, bp);
         break;
       case K_OBJECTIVE:
         k_objective_batch<LAT, S><<<grid, block, 0, st>>>(bp);
@@ -1026,14 +1061,15 @@ struct OpsImpl {
                      double* aux) {
     switch (kind) {
       case K_FORWARD:
-        launch_overlapped(k_forward<LAT, COLL, S>, grid, block, st, p);
-        break;
       case K_ADJOINT:
-        launch_overlapped(k_adjoint<LAT, COLL, S>, grid, block, st, p);
-        break;
       case K_ADJOINT_LEAN:
-        launch_overlapped(k_adjoint<LAT, COLL, S, Occupancy<LAT, COLL, S>::has_lean>, grid, block,
-                          st, p);
+        if constexpr (kFixed<S>) {
+          if (p.fix.ok) {
+            launch_step<true>(kind, grid, block, st, p);
+            break;
+          }
+        }
+        launch_step<false>(kind, grid, block, st, p);
         break;
       case K_OBJECTIVE:
         k_objective<LAT, S><<<grid, block, 0, st>>>(p);

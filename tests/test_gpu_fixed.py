@@ -81,3 +81,27 @@ def test_large_drag_leaves_the_porosity_plane(orc, name):
         f = h.populations()
     fo, _, _ = orc.forward(cfg, gamma, 12)
     assert rel_inf(f, fo) < TOL
+
+
+@pytest.mark.parametrize("n", [60, 420])
+def test_velocity_objective_before_and_after_the_flow_arrives(orc, n):
+    """75x75 pump: the pressure wave takes some 60 steps to the outlets.  Sweeps
+    up to 194 steps keep the FP64 operators, longer ones do not."""
+    cfg = W.pump_2d(75, nsteps=n, period=100.0)
+    gamma, table = W.design_2d(75, 75, 9), W.pump_inflow_profile(cfg)
+    with G.Handle(cfg) as h:
+        h.set_bc_profile(2, table)
+        h.set_design(gamma)
+        h.init_equilibrium()
+        J, js = h.forward(n, per_step=True)
+        Jg, s, _ = h.gradient(n, 10)
+    try:
+        orc.set_tables({2: table})
+        _, jo, _ = orc.forward(cfg, gamma, n)
+        Jgo, so = orc.gradient(cfg, gamma, n)
+    finally:
+        orc.set_tables()
+    # the FP64 velocities drift by about 2e-17 a step
+    drift = 5e-17 * n
+    assert np.abs(js - jo).max() < drift / n and abs(Jg - Jgo) < drift
+    assert np.abs(s - so).max() <= 1e-12 * np.abs(so).max() + drift / n
