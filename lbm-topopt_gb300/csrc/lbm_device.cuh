@@ -1927,10 +1927,13 @@ __device__ __forceinline__ void grid_reduce_v(C v, const KParams& p, unsigned bi
     // a fence nor a barrier is needed and the additions come in a fixed
     // order; warps whose cells contribute nothing (e.g. away from the
     // pressure-drop strips) skip the shuffle tree.  The add's result is
-    // unused, so the warp does not wait for the slot's old value.
-    if (__any_sync(0xffffffffu, v != C(0.))) {
-      v = warp_sum(v);
-      if ((tid & 31) == 0)
+    // unused, so the warp does not wait for the slot's old value.  A lone
+    // contribution (a west or east strip of the pressure drop) needs no tree.
+    const unsigned some = __ballot_sync(0xffffffffu, v != C(0.));
+    if (some != 0u) {
+      const bool one = (some & (some - 1u)) == 0u;
+      if (!one) v = warp_sum(v);
+      if (one ? v != C(0.) : (tid & 31) == 0)
         atomicAdd(&p.partial[(size_t)bid * (size_t)(nthr >> 5) + (size_t)(tid >> 5)], (double)v);
     }
     return;

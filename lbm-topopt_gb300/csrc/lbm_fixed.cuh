@@ -77,6 +77,15 @@ __device__ __forceinline__ double from_int(i64 v) {
 #endif
 }
 
+// leading zeros of v != 0
+__device__ __forceinline__ int clz64(u64 v) {
+#if defined(__CUDA_ARCH__)
+  return __clzll((long long)v);
+#else
+  return __builtin_clzll(v);
+#endif
+}
+
 // v * 2^-k to the nearest double (|v| * 2^-k normal or zero).
 __device__ __forceinline__ double to_double(i64 v, int k) {
   const double d = from_int(v);
@@ -94,6 +103,7 @@ __device__ __forceinline__ u64 umul_top(u64 a, u64 b) {
 }
 
 constexpr u64 kBias = 1ull << 63;
+using u128 = unsigned __int128;
 
 // m * c / 2^64 within two units, c >= 0 and even: (m + 2^63) c / 2^64 - c / 2
 // (unsigned products are the cheap ones).  The truncations lose 1.25 on
@@ -844,13 +854,38 @@ struct Stress2 {
   }
 };
 
-// w (2 alpha j^2 + cv V:V); the products of the small V_ab in FP64
-__device__ __forceinline__ double dissipation2(const i64* x, u64 im, double w, double cv) {
+__device__ __forceinline__ u128 square(i64 a) {
+  const u64 m = (u64)(a < 0 ? -a : a);
+  return (u128)m * m;
+}
+// a * c / 2^64
+__device__ __forceinline__ u128 times(u128 a, u64 c) {
+  return (u128)(u64)(a >> 64) * c + (u64)(((u128)(u64)a * c) >> 64);
+}
+
+// (2 alpha j^2 + cv V:V) * 2^117, cv given * 2^64: below 2^121.  The 128-bit
+// products leave a slow flow's squares (1e-14 at u = 1e-7) their bits, and cost
+// four 32-bit multiplies of 1.4 cycles a warp each where a conversion or a
+// product on the FP64 pipe takes 16.
+constexpr int kEnergyScale = 117;
+__device__ __forceinline__ u128 dissipation2(const i64* x, u64 im, u64 cv) {
   const Stress2 v(x, Pairs2(x));
-  const double xx = to_double(v.xx, kScale), yy = to_double(v.yy, kScale),
-               xy = to_double(v.xy, kScale);
-  const double alpha = to_double((i64)(im >> 1), 63);
-  return w * (2. * (alpha * v.jj()) + cv * ((xx * xx + yy * yy) + 2. * (xy * xy)));
+  const u128 a = times(square(v.qx) + square(v.qy), im);               // * 2^126
+  const u128 b = times(square(v.xx) + square(v.yy) + 2 * square(v.xy), cv);   // * 2^122
+  return (a >> (126 - 1 - kEnergyScale)) + (b >> (122 - kEnergyScale));
+}
+__device__ __forceinline__ double energy(u128 e) {
+  u64 h = (u64)(e >> 64), l = (u64)e;
+  int k = kEnergyScale - 64;
+  if (h == 0ull) {
+    h = l;
+    l = 0ull;
+    k += 64;
+  }
+  if (h == 0ull) return 0.;
+  const int s = clz64(h) - 1;   // as a positive i64
+  h = s >= 0 ? (h << s) | ((l >> 1) >> (63 - s)) : h >> 1;
+  return to_double((i64)h, k + s);
 }
 
 // The objective's derivatives by f and by imult, both over the weight.

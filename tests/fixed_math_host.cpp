@@ -204,7 +204,7 @@ int fixed_dissipation(const lbm_config* c, int n, const double* f, const double*
       x[q] = w.load<LAT_D2Q9, q>(f[i * 9 + q]);
     });
     if (!w.ok<LAT_D2Q9>(x)) return i;
-    val[i] = fx::dissipation2(x, im, c->obj_weight, p.md.cv_diss);
+    val[i] = c->obj_weight * fx::energy(fx::dissipation2(x, im, p.fix.cv));
     for (int k = 0; k < 9; ++k) src[9 * i + k] = src64[9 * i + k] = 0.;
     const fx::Dissipation2 d(x, fx::Factor(im), p.fix.cv);
     dim[i] = d.dim;

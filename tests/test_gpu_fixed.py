@@ -105,3 +105,35 @@ def test_velocity_objective_before_and_after_the_flow_arrives(orc, n):
     drift = 5e-17 * n
     assert np.abs(js - jo).max() < drift / n and abs(Jg - Jgo) < drift
     assert np.abs(s - so).max() <= 1e-12 * np.abs(so).max() + drift / n
+
+
+@pytest.mark.parametrize("objective,box", [
+    (G.OBJ_DISSIPATION, None),
+    (G.OBJ_PRESSURE_DROP, (0, 0, 1, 38, 0, 0)),      # one lane of a warp
+    (G.OBJ_PRESSURE_DROP, (0, 40, 7, 7, 0, 0)),      # a full warp and a part of one
+    (G.OBJ_PRESSURE_DROP, (31, 32, 3, 3, 0, 0)),     # one lane each of two warps
+])
+@pytest.mark.parametrize("amp", [0.0, 1e-7, 0.05])
+def test_sums_over_the_warp(orc, objective, box, amp):
+    """Objectives that all, some or single lanes of a warp contribute to, from a
+    fluid at rest, a slow and a fast flow; J of a sweep and of its steps."""
+    nx, ny, n = 41, 40, 9
+    cfg = W.channel_2d(nx, ny, nsteps=n, objective=objective)
+    if box:
+        cfg = cfg.replace(obj_in=box)
+    gamma = W.design_2d(nx, ny, 5)
+    mac = np.zeros((nx * ny, 3))
+    mac[:, 0] = 1.0
+    mac[:, 1:] = amp * np.random.default_rng(3).uniform(-1, 1, (nx * ny, 2))
+    with G.Handle(cfg) as h:
+        h.set_design(gamma)
+        h.init_equilibrium(mac)
+        _, js = h.forward(n, per_step=True)
+        h.init_equilibrium(mac)
+        J, _, _ = h.gradient(n, 3)
+    _, jo, _ = orc.forward(cfg, gamma, n, macros=mac)
+    # a step's J adds up to nx ny values of the size of its largest cell's, whose
+    # own roundings are a few 2^-53 of a density (pressure) or of j^2 and V^2
+    size = np.abs(jo).max() if objective == G.OBJ_DISSIPATION else 1.0 / n
+    assert np.abs(js - jo).max() <= 1e-13 * size
+    assert abs(J - jo.sum()) <= 1e-13 * size * n
