@@ -125,6 +125,7 @@ const int kBlockThreads = 256;
 struct Geometry {
   dim3 grid, block;
   unsigned nblocks;
+  size_t threads() const { return (size_t)nblocks * block.x * block.y; }
 };
 
 Geometry make_geometry(int nx, int ny, int nz, int bx, int by) {
@@ -141,6 +142,50 @@ Geometry make_geometry(int nx, int ny, int nz, int bx, int by) {
 // forward and 12.3 -> 11.4 us reverse).
 const int kShapes[][2] = {{256, 1}, {128, 2}, {64, 4}, {32, 8}, {128, 1}, {64, 2}, {32, 4},
                           {64, 1}, {32, 2}};
+
+// x-major block of `threads` threads over rows of nx cells
+Geometry row_blocks(const lbm_config& c, int nz, int threads) {
+  const int row = ((c.nx + 31) / 32) * 32, bx = row < threads ? row : threads;
+  return make_geometry(c.nx, c.ny, nz, bx, threads / bx);
+}
+
+// Whether that many threads are more than the forward step keeps resident at
+// once (Occupancy in lbm_kernels.cuh).
+bool past_one_wave(const lbm_config& c, size_t threads, int nsm) {
+  const int blocks = c.storage == LBM_STORE_FP64 ? 2 : c.lattice == LBM_D2Q9 ? 6 : 5;
+  return threads > (size_t)nsm * blocks * 256;
+}
+
+// Block shape of the step kernels of a handle that is not tuned, by the number
+// of 256-thread blocks of whole rows (times in us forward / reverse, from that
+// shape to the one taken).
+Geometry default_geometry(const lbm_config& c, int nz, int nsm) {
+  const Geometry wide = row_blocks(c, nz, 256);
+  const bool fp64 = c.storage == LBM_STORE_FP64;
+  Geometry g = wide;
+  if (wide.nblocks <= (unsigned)nsm / 2) {
+    // Half the SMs would stay idle: 64 threads a block.  FP64 128x64 5.3 / 7.2 to
+    // 4.2 / 6.4, 64x48 5.9 / 8.7 to 4.2 / 6.8, duct 32x16x16 11.0 / 18.0 to
+    // 7.5 / 12.5; FP32 128x64 3.1 / 3.4 to 2.7 / 2.8, thermal 128x64 3.5 / 4.6 to
+    // 2.9 / 3.7.
+    g = row_blocks(c, nz, 64);
+  } else if (fp64 && c.lattice == LBM_D3Q19) {
+    // The cells of the west and east faces, with their boundaries and objective,
+    // are the long ones, and rows spread them over every block.  256x128x128
+    // 398 / 648 to 306 / 569, 250x121x115 341 / 551 to 267 / 491, 64x32x32
+    // 16.7 / 26.6 to 12.8 / 23.8.
+    g = make_geometry(c.nx, c.ny, nz, 32, 4);
+  } else if (wide.nblocks > (unsigned)nsm * (fp64 ? 2 : 4)) {
+    // Past two (FP64) or four resident blocks per SM, those of the larger step
+    // kernels, 128 threads leave a shorter last wave: FP64 640x240 8.4 / 14.3 to
+    // 7.7 / 13.4, 2048x1024 68 / 123 to 64 / 112; FP32 640x240 4.1 / 5.2 to
+    // 3.9 / 4.4, 1024x512 9.6 / 12.3 to 8.2 / 10.2, duct 256x128x128 114.8 / 163.3
+    // to 110.6 / 158.2.  Fewer blocks stay at 256: FP64 thermal 255x97 5.7 / 10.1
+    // against 5.9 / 11.4, FP32 400x200 3.31 / 3.81 against 3.36 / 3.83.
+    g = row_blocks(c, nz, 128);
+  }
+  return g.grid.y <= 65535u ? g : wide;   // the grid's limit along y
+}
 
 }  // namespace
 
@@ -162,6 +207,7 @@ struct lbm_handle {
   bool adj_wide = false;   // FP64 D2Q9 reverse step with three resident blocks (wide_reverse)
   bool sens_atomic = false;   // reverse step adds to dJ/dgamma atomically (fits in L2)
   bool tuned = false;
+  int nsm = 1;
   size_t partial_cap = 0;
   void* f[2] = {nullptr, nullptr};
   int cur = 0;
@@ -468,6 +514,8 @@ KParams base_params(const lbm_handle* h, int t) {
   p.step = (unsigned)t;
   p.key_fwd = step_key(p.step, kSaltForward);
   p.key_adj = step_key(p.step, kSaltAdjoint);
+  p.early_fwd = past_one_wave(c, h->geo_fwd.threads(), h->nsm);
+  p.early_adj = past_one_wave(c, h->geo_adj.threads(), h->nsm);
   p.omega = c.omega;
   for (int i = 0; i < 8; ++i) p.mrt[i] = c.mrt[i];
   p.pbb_scale = c.interp_scale;
@@ -836,14 +884,13 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
     return fail(nullptr, LBM_ERR_SUP, "no kernel for lattice %d collision %d storage %d", lat, coll,
                 stor);
   }
-  // thread blocks: 256 threads, x-major rows
-  int bx = c.nx >= 256 ? 256 : ((c.nx + 31) / 32) * 32;
-  if (bx > 256) bx = 256;
-  int by = kBlockThreads / bx;
-  if (by < 1) by = 1;
-  h->geo = make_geometry(c.nx, c.ny, h->cfg.nz, bx, by);
-  h->geo_fwd = h->geo;
-  h->geo_adj = h->geo;
+  h->geo = row_blocks(c, h->cfg.nz, kBlockThreads);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    h->nsm = 1;
+  h->geo_fwd = default_geometry(c, h->cfg.nz, h->nsm);
+  h->geo_adj = h->geo_fwd;
   // partial sums: one slot per warp of the largest grid any tuned shape gives
   for (const auto& sh : kShapes) {
     Geometry g = make_geometry(c.nx, c.ny, h->cfg.nz, sh[0], sh[1]);
@@ -1834,6 +1881,7 @@ void batch_layout(lbm_batch* b, BatchParams& bp, int kind) {
   // slots past the batch start at the total (the kernels count the starts
   // at or below a block)
   for (int i = b->n; i <= kMaxBatch; ++i) bp.start[i] = start;
+  bp.early = past_one_wave(b->h[0]->cfg, (size_t)start * blk.x * blk.y, b->nsm);
 }
 
 // Persistent grids of the batched kernels for the current block shapes.
@@ -2109,8 +2157,11 @@ int lbm_batch_create(const lbm_config* cfgs, int n, lbm_batch** out) {
       return bfail(nullptr, LBM_ERR_CUDA, "batch set-up failed: cudaEventCreate");
     }
   }
-  // default shapes: 128x2, one of the autotuner's shapes (partial sums are sized for all)
-  b->bx = b->abx = 128;
+  // default shape, one of the autotuner's (partial sums are sized for all), in us
+  // forward / reverse for the 8 channels and for a quarter of their edges, from
+  // 128x2: FP32 39.2 / 61.0 to 37.6 / 56.7 and 7.1 / 7.9 to 6.6 / 5.6, FP64
+  // 85.1 / 152.3 to 78.6 / 138.0 and 12.9 / 17.2 to 12.7 / 17.4.
+  b->bx = b->abx = 64;
   b->by = b->aby = 2;
   batch_set_grids(b);
   b->grid_copy = 4 * b->nsm;

@@ -718,16 +718,31 @@ __device__ __forceinline__ typename Store<S>::C objective_only_cell(const KParam
 // Start of every time-step kernel.  The step kernels are launched with
 // programmatic stream serialisation (launch_overlapped): their CTAs may be
 // scheduled while the previous kernel in the stream drains its last wave.
-// Each CTA lets the next launch proceed, then waits until the previous grid
-// has completed and its writes are visible, before it touches memory.
-__device__ __forceinline__ void step_prologue() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// Each CTA waits until the previous grid has completed and its writes are
+// visible, before it touches memory.
+// When it lets the next launch proceed depends on the grid.  Early (before the
+// wait) the grids of several steps to come line up on the SMs; where one wave
+// does not fill the chip, their waiting CTAs take the places that would have
+// spread the running step's CTAs evenly, and some SMs get twice the others'.
+// So FP64 steps let it proceed after the wait (at most one grid waits: 256x140
+// 6.4 / 8.4 to 4.3 / 6.7 us forward / reverse, thermal 255x97 7.6 / 16.8 to
+// 5.6 / 11.1, larger grids within 0.3%), and FP32 and FP16 grids of one wave not
+// before their CTAs end (FP32 512x256 5.2 / 4.9 to 3.8 / 4.4, 64x32x32 7.0 / 6.8
+// to 5.0 / 4.7, thermal 255x97 3.4 / 6.6 to 2.8 / 3.9; after the wait 5.0 / 4.6,
+// 5.0 / 4.7, 3.2 / 4.1).  Larger FP32 and FP16 grids keep the early launch: the
+// FP16 100x60x60 duct's reverse step is 15.2 us with it and 16.0 without.
+template <class S>
+__device__ __forceinline__ void step_prologue(int early) {
+  if (!std::is_same<S, double>::value && early)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (std::is_same<S, double>::value)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <int LAT, int COLL, class S, bool FIXED = false>
 __global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S, FIXED>::fwd) k_forward(KParams p) {
-  step_prologue();
+  step_prologue<S>(p.early_fwd);
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   constexpr bool W = kWarpInterior<LAT>;
@@ -745,7 +760,7 @@ template <int LAT, int COLL, class S, bool LEAN = false, bool FIXED = false>
 __global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S, FIXED>::adj_lean
                                             : Occupancy<LAT, COLL, S, FIXED>::adj)
     k_adjoint(KParams p) {
-  step_prologue();
+  step_prologue<S>(p.early_adj);
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   constexpr bool W = kWarpInterior<LAT>;
@@ -781,7 +796,7 @@ __device__ __forceinline__ int batch_lattice_of(const BatchParams& bp, int vb) {
 template <int LAT, int COLL, class S, bool FIXED = false>
 __global__ void __launch_bounds__(256, Occupancy<LAT, COLL, S, FIXED>::fwd)
     k_forward_batch(const __grid_constant__ BatchParams bp) {
-  step_prologue();
+  step_prologue<S>(bp.early);
   for (int vb = blockIdx.x; vb < bp.start[kMaxBatch]; vb += gridDim.x) {
     const int i = batch_lattice_of(bp, vb);
     const KParams& p = bp.p[i];
@@ -815,7 +830,7 @@ template <int LAT, int COLL, class S, bool LEAN = false, bool FIXED = false>
 __global__ void __launch_bounds__(256, LEAN ? Occupancy<LAT, COLL, S, FIXED>::adj_lean_batch
                                             : Occupancy<LAT, COLL, S, FIXED>::adj)
     k_adjoint_batch(const __grid_constant__ BatchParams bp) {
-  step_prologue();
+  step_prologue<S>(bp.early);
   for (int vb = blockIdx.x; vb < bp.start[kMaxBatch]; vb += gridDim.x) {
     const int i = batch_lattice_of(bp, vb);
     const KParams& p = bp.p[i];
