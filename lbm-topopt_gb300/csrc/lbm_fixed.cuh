@@ -95,6 +95,19 @@ __device__ __forceinline__ double to_double(i64 v, int k) {
 
 // --- products ----------------------------------------------------------------
 
+// A product kept apart from the sums it enters.  Without this the compiler
+// gathers the subtracted halves of several signed products into one sum and
+// drops the carry of its subtraction where the sum's low word is zero: one reverse
+// step in about 2^31 came out wrong by 2^32 units (4e-8 of a population of the
+// cell).  Over 1e10 to 4e10 random cells per model and direction against the FP64
+// operators: up to 21 such cells without it, none with it.
+__device__ __forceinline__ i64 apart(i64 v) {
+#if defined(__CUDA_ARCH__)
+  asm("" : "+l"(v));
+#endif
+  return v;
+}
+
 // The top 64 bits of a * b without the low partial product and the carries of
 // the middle ones: short of the exact quotient by less than 3.
 __device__ __forceinline__ u64 umul_top(u64 a, u64 b) {
@@ -109,7 +122,7 @@ using u128 = unsigned __int128;
 // (unsigned products are the cheap ones).  The truncations lose 1.25 on
 // average, of which 1 is added back: a quarter too low in the mean.
 __device__ __forceinline__ i64 mulc(i64 m, u64 c) {
-  return (i64)umul_top((u64)m ^ kBias, c) - (i64)(c >> 1) + 1;
+  return apart((i64)umul_top((u64)m ^ kBias, c) - (i64)(c >> 1) + 1);
 }
 // A cell's own factor c, with the constant part of mulc prepared: a factor of
 // zero (fluid) gives exactly zero, so that nothing is added to the momentum of
@@ -119,18 +132,18 @@ struct Factor {
   i64 k;
   __device__ __forceinline__ explicit Factor(u64 v) : c(v), k((i64)(v >> 1) - (v != 0ull ? 1 : 0)) {}
   __device__ __forceinline__ i64 times(i64 m) const {
-    return (i64)umul_top((u64)m ^ kBias, c) - k;
+    return apart((i64)umul_top((u64)m ^ kBias, c) - k);
   }
 };
 // a * b / 2^64 and a * a / 2^64 for signed operands: (a + 2^63)(b + 2^63) =
 // a b + 2^63 (a + b) + 2^126.
 __device__ __forceinline__ i64 mulr(i64 a, i64 b) {
-  return (i64)umul_top((u64)a ^ kBias, (u64)b ^ kBias) - ((a >> 1) + (b >> 1)) -
-         ((1ll << 62) - 1);
+  return apart((i64)umul_top((u64)a ^ kBias, (u64)b ^ kBias) - ((a >> 1) + (b >> 1)) -
+               ((1ll << 62) - 1));
 }
 __device__ __forceinline__ i64 sqr(i64 a) {
   const u64 u = (u64)a ^ kBias;
-  return (i64)umul_top(u, u) - a - ((1ll << 62) - 1);
+  return apart((i64)umul_top(u, u) - a - ((1ll << 62) - 1));
 }
 // m * c for a signed constant |c| < 2 given as |c| 2^62 and its sign (0, -1).
 __device__ __forceinline__ i64 muls(i64 m, u64 c, int neg) {
@@ -319,6 +332,15 @@ struct BlockOf {
     zero = m == 0u;
     ok = top >= 323 && top <= 1077;
     k = 1022 + BITS - top;
+  }
+  // no finer than 2^-kmax
+  __device__ __forceinline__ void at_most(int kmax) {
+    if (zero || k > kmax) {
+      k = kmax;
+      top = 1022 + BITS - k;
+      zero = false;
+      ok = true;
+    }
   }
   // v * 2^k rounded to the nearest integer.  The conversion runs on the FP64
   // pipe, except that the temperature lattice, whose two scales and FP64 terms
@@ -911,9 +933,23 @@ struct Dissipation2 {
     src.ev[4] = mulc((v.xx - t3) << 1, c);
     dim = 2. * v.jj();
   }
+  // The finest scale of a Block whose units take the source times the weight
+  // (scaled): its error, some units of w 2^-61, is far above 2^-89 w.  Where the
+  // adjoint is much smaller than the source (the first reverse steps, a fluid at
+  // rest) its own finer units would not: such cells took an FP64 sum until then,
+  // and a 2048x1024 reverse step whose flow had not developed 200 us, now 141.
+  __device__ __forceinline__ int scale_limit(const FixedModel& m) const {
+    const i64 v[7] = {src.ev[0], src.ev[1], src.ev[2], src.ev[3], src.ev[4], src.gx, src.gy};
+    u64 any = 1u;
+    static_for<7>([&](auto I) {
+      const i64 t = v[decltype(I)::value];
+      any |= (u64)(t ^ (t >> 63));
+    });
+    const int sh = clz64(any) - 5;   // one bit for the product's rounding
+    return 64 - m.w_exp + (sh < 27 ? sh : 27);
+  }
   // the source times the weight in the units of a Block's results, where that
-  // fits (on): it does unless the adjoint is much smaller than the weight, as
-  // in the first reverse steps
+  // fits (on)
   __device__ __forceinline__ Source2 scaled(const FixedModel& m, const Block& b) const {
     Source2 r;
     const int sh = m.w_exp + b.k - 64;
@@ -936,17 +972,6 @@ struct Dissipation2 {
     r.gx = v[5];
     r.gy = v[6];
     return r;
-  }
-  // lam += w dF/df in FP64
-  __device__ __forceinline__ void add(double w, double* lam) const {
-    const double w61 = w * 4.336808689942017736029811203479766845703125e-19;   // w 2^-61
-    lam[0] += w61 * from_int(src.ev[0]);
-    static_for<4>([&](auto D) {
-      constexpr int k = decltype(D)::value + 1;
-      const i64 eg = e_dot<LAT_D2Q9, k>(src.gx, src.gy, (i64)0);
-      lam[k] += w61 * from_int(src.ev[k] + eg);
-      lam[k + 4] += w61 * from_int(src.ev[k] - eg);
-    });
   }
 };
 

@@ -308,12 +308,6 @@ __device__ __noinline__ void reverse_fp64(const double* f, double* lam, double g
   }
 }
 
-// The dissipation's source onto the adjoint of a cell whose units do not take it.
-static __device__ __noinline__ void add_dissipation_fp64(const fx::i64* x, unsigned long long im,
-                                                  const KParams& p, double* lam) {
-  fx::Dissipation2(x, fx::Factor(im), p.fix.cv).add(p.md.obj_weight, lam);
-}
-
 // Whether the collision can run in fixed point: FP64 storage.  The step kernels
 // are built twice for it: FIXED ones, in which cells (and, in a batch, whole
 // lattices) may still take the FP64 operators, and FP64 ones without the
@@ -547,13 +541,14 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
       xi[q] = w.template load<LAT, q>(f[q]);
     });
     ok = ok && w.template ok<LAT>(xi) && des.ok();
-      if (ok) {
+    if (ok) {
       const fx::Factor im(des.im);
       fx::Source2 src;
       double ddiss = 0.;
       if constexpr (L::DIM == 2) {
         if (diss) {
           const fx::Dissipation2 d(xi, im, p.fix.cv);
+          b.at_most(d.scale_limit(p.fix));
           src = d.scaled(p.fix, b);
           ddiss = dimult * (p.md.obj_weight * d.dim);
         }
@@ -562,22 +557,7 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
       if constexpr (THERMAL) {
         if (!l.zero) dg += thermal_reverse_cell(p, c, f, lam, fx::Pairs2(xi), g, l, des.om6);
       }
-      if constexpr (L::DIM == 2) {
-        if (diss) {
-          dg += ddiss;
-          if (!src.on) {
-            fx::i64 xs[L::QF];
-            double s[L::QF];
-            static_for<L::QF>([&](auto Q_) {
-              constexpr int q = decltype(Q_)::value;
-              xs[q] = xi[q];
-              s[q] = lam[q];
-            });
-            add_dissipation_fp64(xs, des.im, p, s);
-            static_for<L::QF>([&](auto Q_) { lam[decltype(Q_)::value] = s[decltype(Q_)::value]; });
-          }
-        }
-      }
+      dg += ddiss;
     } else {
       double t[L::Q], u[L::Q], d = 0.;
       static_for<L::Q>([&](auto Q_) {

@@ -224,7 +224,20 @@ int fixed_dissipation(const lbm_config* c, int n, const double* f, const double*
         src[9 * i + k + 4] = b.store(r.ev[k] - eg);
       });
     } else {
-      d.add(c->obj_weight, src + 9 * i);
+      // beside an adjoint of zero, as in units that take it
+      fx::Block z;
+      const double none[1] = {0.};
+      z.measure<1>(none);
+      z.at_most(d.scale_limit(p.fix));
+      const fx::Source2 r0 = d.scaled(p.fix, z);
+      if (!r0.on) return i;
+      src[9 * i] = z.store(r0.ev[0]);
+      static_for<4>([&](auto D) {
+        constexpr int k = decltype(D)::value + 1;
+        const fx::i64 eg = e_dot<LAT_D2Q9, k>(r0.gx, r0.gy, (fx::i64)0);
+        src[9 * i + k] = z.store(r0.ev[k] + eg);
+        src[9 * i + k + 4] = z.store(r0.ev[k] - eg);
+      });
     }
     val64[i] = ObjDissipation::evaluate<LAT_D2Q9, false>(f + 9 * i, g[i], 0, 0, 0, p);
     double dg = 0.;

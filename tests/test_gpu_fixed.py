@@ -137,3 +137,28 @@ def test_sums_over_the_warp(orc, objective, box, amp):
     size = np.abs(jo).max() if objective == G.OBJ_DISSIPATION else 1.0 / n
     assert np.abs(js - jo).max() <= 1e-13 * size
     assert abs(J - jo.sum()) <= 1e-13 * size * n
+
+
+@pytest.mark.parametrize("collision", [G.BGK, G.MRT])
+def test_dissipation_adjoint_of_a_fluid_at_rest(collision):
+    """Cells that the flow has not reached: every product of the source and of
+    the transposed collision has a zero operand, and the adjoint has to stay
+    within the units of 2^-61 of the weight that the products may lose (some
+    tens of them a step; a lost carry is 2^32 of them)."""
+    nx, ny, n = 160, 40, 4
+    cfg = W.channel_2d(nx, ny, nsteps=n, objective=G.OBJ_DISSIPATION, collision=collision)
+    with G.Handle(cfg) as h:
+        h.set_design(W.design_2d(nx, ny, 6))
+        h.init_equilibrium()
+        states = []
+        for t in range(1, n + 1):
+            h.forward(1)
+            states.append(h.populations())
+        h.adjoint_reset()
+        for t in range(n, 0, -1):
+            h.set_populations(states[t - 1], t)
+            h.adjoint_step()
+        lam = h.adjoint().reshape(ny, nx, 9)
+    far = lam[8:-8, 20:-20]
+    assert np.abs(far).max() <= 1000 * n * 2.0 ** -61 * abs(cfg.obj_weight)
+    assert np.abs(lam).max() > 1e-9 * abs(cfg.obj_weight)
