@@ -18,6 +18,7 @@
 #include "../../include/lbmgpu.h"
 #include "fixed_model.hpp"
 #include "host_buffers.hpp"
+#include "mapped_slots.hpp"
 #include "lbm_device.cuh"
 #include "lbm_ops.h"
 #include "state_pool.hpp"
@@ -476,8 +477,8 @@ void destroy_buffers(lbm_handle* h) {
   for (void* s : h->slots)
     if (s) cudaFree(s);
   h->slots.clear();
-  void* ps[] = {h->gamma,  h->im,      h->dimult,  h->om6,  h->domega, h->sens,
-                h->partial, h->counter, h->jdev, h->stage, h->init_mac, h->step_partial};
+  void* ps[] = {h->gamma,   h->sens,  h->partial,  h->counter,
+                h->jdev,    h->stage, h->init_mac, h->step_partial};
   for (void* p : ps)
     if (p) cudaFree(p);
   for (int k = 0; k < LBM_MAX_BC; ++k) {
@@ -492,7 +493,7 @@ void destroy_buffers(lbm_handle* h) {
   h->om6 = nullptr;
   h->counter = nullptr;
   h->jdev = h->stage = h->init_mac = h->step_partial = nullptr;
-  if (h->jhost) cudaFreeHost(h->jhost);
+  if (h->jhost) MappedSlots::give(h->jhost);   // the stream's work is done
   h->jhost = h->jhost_dev = nullptr;
   for (cudaEvent_t& e : h->ev)
     if (e) {
@@ -640,10 +641,10 @@ constexpr int64_t kDeviceCheck = 8192;
 
 int ensure_jhost(lbm_handle* h) {
   if (h->jhost) return 0;
-  double* v = nullptr;
-  CUDA_OR_FAIL(h, cudaHostAlloc((void**)&v, 2 * sizeof(double), cudaHostAllocMapped));
-  h->jhost = v;
-  CUDA_OR_FAIL(h, cudaHostGetDevicePointer((void**)&h->jhost_dev, v, 0));
+  cudaError_t e = cudaSuccess;
+  h->jhost = (double*)MappedSlots::take(&e);
+  CUDA_OR_FAIL(h, e);
+  CUDA_OR_FAIL(h, cudaHostGetDevicePointer((void**)&h->jhost_dev, h->jhost, 0));
   return 0;
 }
 
@@ -928,15 +929,19 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   ALLOC(h->f[1], state_bytes(h));
   ALLOC(h->lam[0], adjoint_bytes(h));
   ALLOC(h->lam[1], adjoint_bytes(h));
-  ALLOC(h->gamma, (size_t)h->P * h->gam_bytes);
   h->fix = fixed_model(c);
   h->start_up = flow_start_up(c);
-  if (h->fix.ok) {
-    ALLOC(h->im, (size_t)h->P * sizeof(unsigned long long));
-    ALLOC(h->dimult, (size_t)h->P * sizeof(double));
-    if (c.lattice == LBM_D2Q9_D2Q5) {
-      ALLOC(h->om6, (size_t)h->P * sizeof(unsigned long long));
-      ALLOC(h->domega, (size_t)h->P * sizeof(double));
+  // the design's planes: gamma and, of 8 bytes a cell as well (FP64 storage),
+  // those of the fixed-point collisions
+  const int planes = !h->fix.ok ? 1 : c.lattice == LBM_D2Q9_D2Q5 ? 5 : 3;
+  ALLOC(h->gamma, (size_t)h->P * h->gam_bytes * planes);
+  if (planes >= 3) {
+    double* plane = (double*)h->gamma;
+    h->im = (unsigned long long*)(plane += h->P);
+    h->dimult = plane += h->P;
+    if (planes == 5) {
+      h->om6 = (unsigned long long*)(plane += h->P);
+      h->domega = plane += h->P;
     }
   }
   ALLOC(h->sens, (size_t)h->P * sizeof(double));

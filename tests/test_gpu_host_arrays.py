@@ -67,3 +67,34 @@ def test_results_in_any_host_memory(nx, ny):
             h._check(h.lib.lbm_get_populations(h.h, p))
             assert np.array_equal(keep[off:off + n], f)
             assert (keep[:off] == 7.0).all() and (keep[off + n:] == 7.0).all()
+
+
+def test_results_of_many_handles_in_threads():
+    """Handles share pages of 64 result slots: more than two pages' worth alive at
+    once, used from four threads, closed and made again."""
+    import threading
+    import workloads as W
+    cfg = W.channel_2d(20, 12, nsteps=4)
+    designs = [W.design_2d(20, 12, 50 + k) for k in range(140)]
+
+    def value(h, k):
+        h.set_design(designs[k])
+        h.init_equilibrium()
+        return h.forward(4)
+    with G.Handle(cfg) as h:
+        want = [value(h, k) for k in range(140)]
+    got = [[None] * 140 for _ in range(2)]
+
+    def work(part):
+        for turn in range(2):
+            hs = {k: G.Handle(cfg) for k in range(part, 140, 4)}
+            for k, x in hs.items():
+                got[turn][k] = value(x, k)
+            for x in hs.values():
+                x.close()
+    threads = [threading.Thread(target=work, args=(p,)) for p in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got[0] == want and got[1] == want
