@@ -55,8 +55,9 @@ extern "C" {
 #define LBM_MRT 1   /* IncompressibleMRT2d / IncompressibleMRT3d (dynamics/MRT3d.hh:28-200) */
 
 /* Population storage in device memory.  Compute precision is FP64 for
- * LBM_STORE_FP64 and FP32 for the two shifted forms, which store the
- * deviation f_i - w_i. */
+ * LBM_STORE_FP64 (collisions of cells near equilibrium in 64-bit fixed point,
+ * with a smaller error than the FP64 expressions) and FP32 for the two shifted
+ * forms, which store the deviation f_i - w_i. */
 #define LBM_STORE_FP64 0
 #define LBM_STORE_FP32 1
 #define LBM_STORE_FP16 2

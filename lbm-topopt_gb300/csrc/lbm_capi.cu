@@ -138,9 +138,8 @@ Geometry make_geometry(int nx, int ny, int nz, int bx, int by) {
 }
 
 // Thread-block shapes the autotuner tries (x-major rows; 64, 128 or 256
-// threads: the 64-thread ones spread lattices of a few thousand blocks more
-// evenly over the SMs, e.g. the 128x64 FP64 channel's steps 6.2 -> 5.6 us
-// forward and 12.3 -> 11.4 us reverse).
+// threads: the 64-thread ones put lattices of a few thousand cells on all SMs,
+// see default_geometry).
 const int kShapes[][2] = {{256, 1}, {128, 2}, {64, 4}, {32, 8}, {128, 1}, {64, 2}, {32, 4},
                           {64, 1}, {32, 2}};
 

@@ -19,11 +19,15 @@
 // lbm_device.cuh, cell by cell, as do models whose constants do not fit
 // (FixedModel::ok).
 //
-// Measured on one GB300, FP64 -> fixed point: 256x128x128 D3Q19 MRT step 1.916
-// -> 0.282 ms forward (4.7 TB/s, 0.70 of the copy bandwidth) and 3.081 ->
-// 0.717 ms reverse; 4096x2048 D2Q9 BGK 1.457 -> 0.208 ms (6.1 TB/s, 0.92) and
-// 2.907 -> 0.329 ms; 2048x1024 D2Q9 MRT 0.561 -> 0.055 ms and 1.243 -> 0.089
-// ms; 128x64 BGK 5.6 -> 3.6 us and 11.1 -> 6.2 us.  Root-mean-square error of
+// Measured on one GB300 with the objective, over flows and adjoints that fill
+// the lattice, FP64 -> fixed point: 256x128x128 D3Q19 MRT step 1.916 -> 0.309 ms
+// forward (4.2 TB/s, 0.63 of the copy bandwidth; 0.289 without the objective)
+// and 3.081 -> 0.569 ms reverse; 4096x2048 D2Q9 BGK 1.457 -> 0.238 ms (5.4 TB/s,
+// 0.80) and 2.907 -> 0.408 ms; 2048x1024 D2Q9 MRT 0.561 -> 0.064 ms and 1.243 ->
+// 0.110 ms; 128x64 BGK 5.6 -> 4.2 us and 11.1 -> 6.3 us.  Where no adjoint has
+// arrived the reverse step only reads it (256x128x128 0.419 ms in the first 30
+// steps).  What bounds them is the integer pipes' issue and, in the D3Q19 reverse
+// step at 128 registers, too few warps (8 of 64).  Root-mean-square error of
 // one collision against extended precision, over the FP64 operators' own:
 // 0.14 to 0.40 forward, 0.19 to 0.69 reverse.
 #pragma once

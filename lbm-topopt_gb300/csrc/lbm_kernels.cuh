@@ -28,8 +28,7 @@ namespace lbm {
 // forward step fits 6 (42 registers, no spills: 4096x2048 step 0.1079 ->
 // 0.1025 ms, the 8-channel batch's 0.0342 -> 0.0324 ms; 7 spills and is
 // slower); the D3Q19 BGK adjoint in increment form needs more registers than
-// 64 and gets 3 blocks (85); the FP64 kernels are FP64-throughput-bound on
-// GB300 and keep all their registers.
+// 64 and gets 3 blocks (85).  FP64 kernels: below.
 template <int LAT, int COLL, class S, bool FIXED = false>
 struct Occupancy {
   static constexpr int fwd = (LAT == LAT_D2Q9) ? 6 : 5;
