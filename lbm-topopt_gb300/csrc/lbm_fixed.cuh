@@ -26,8 +26,9 @@
 // 0.80) and 2.907 -> 0.408 ms; 2048x1024 D2Q9 MRT 0.561 -> 0.064 ms and 1.243 ->
 // 0.110 ms; 128x64 BGK 5.6 -> 4.2 us and 11.1 -> 6.3 us.  Where no adjoint has
 // arrived the reverse step only reads it (256x128x128 0.419 ms in the first 30
-// steps).  What bounds them is the integer pipes' issue and, in the D3Q19 reverse
-// step at 128 registers, too few warps (8 of 64).  Root-mean-square error of
+// steps).  What bounds them is the FP64 pipe's conversions (54 to 78% busy, two a
+// population) beside the integer work, at 15 to 21 of 64 warps per SM; doubles
+// built on the integer pipes instead were slower.  Root-mean-square error of
 // one collision against extended precision, over the FP64 operators' own:
 // 0.14 to 0.40 forward, 0.19 to 0.69 reverse.
 #pragma once
