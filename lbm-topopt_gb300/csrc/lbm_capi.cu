@@ -159,7 +159,7 @@ bool past_one_wave(const lbm_config& c, size_t threads, int nsm) {
 // Block shape of the step kernels of a handle that is not tuned, by the number
 // of 256-thread blocks of whole rows (times in us forward / reverse, from that
 // shape to the one taken).
-Geometry default_geometry(const lbm_config& c, int nz, int nsm) {
+Geometry default_geometry(const lbm_config& c, int nz, int nsm, bool reverse) {
   const Geometry wide = row_blocks(c, nz, 256);
   const bool fp64 = c.storage == LBM_STORE_FP64;
   Geometry g = wide;
@@ -183,6 +183,15 @@ Geometry default_geometry(const lbm_config& c, int nz, int nsm) {
     // to 110.6 / 158.2.  Fewer blocks stay at 256: FP64 thermal 255x97 5.7 / 10.1
     // against 5.9 / 11.4, FP32 400x200 3.31 / 3.81 against 3.36 / 3.83.
     g = row_blocks(c, nz, 128);
+    // The reverse steps of FP32 and FP16 ducts pull from neighbour rows, which
+    // the four rows of a 32x4 block share in L1: FP32 MRT 256x128x128 159.4 to
+    // 155.9, 128x64x64 24.8 to 22.5, BGK 224x120x90 115.7 to 104.3, FP16 MRT
+    // 256x128x128 151.5 to 148.5.  Where rows do not split into full warps the
+    // two are level (250x121x115 133.8 and 133.9) or rows ahead (100x60x60 15.9
+    // against 16.1), as they are against the 64x2 blocks of rows of 64 (FP16
+    // 64x100x90 26.0 against 26.4).
+    if (reverse && c.lattice == LBM_D3Q19 && c.nx % 32 == 0 && c.nx > 64)
+      g = make_geometry(c.nx, c.ny, nz, 32, 4);
   }
   return g.grid.y <= 65535u ? g : wide;   // the grid's limit along y
 }
@@ -889,8 +898,8 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     h->nsm = 1;
-  h->geo_fwd = default_geometry(c, h->cfg.nz, h->nsm);
-  h->geo_adj = h->geo_fwd;
+  h->geo_fwd = default_geometry(c, h->cfg.nz, h->nsm, false);
+  h->geo_adj = default_geometry(c, h->cfg.nz, h->nsm, true);
   // partial sums: one slot per warp of the largest grid any tuned shape gives
   for (const auto& sh : kShapes) {
     Geometry g = make_geometry(c.nx, c.ny, h->cfg.nz, sh[0], sh[1]);

@@ -41,7 +41,8 @@ def test_2d_bits(nx, ny, storage):
 
 
 @pytest.mark.parametrize("storage", [G.STORE_FP64, G.STORE_FP32, G.STORE_FP16])
-@pytest.mark.parametrize("dims", [(3, 3, 3), (32, 16, 16), (33, 17, 38), (70, 20, 40)])
+@pytest.mark.parametrize("dims", [(3, 3, 3), (32, 16, 16), (33, 17, 38), (70, 20, 40), (64, 64, 41), (96, 63, 41),
+                                  (97, 63, 41)])
 def test_3d_bits(dims, storage):
     n = 5
     cfg = W.duct_3d(*dims, storage=storage, nsteps=n)
