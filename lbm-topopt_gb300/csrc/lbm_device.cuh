@@ -408,7 +408,7 @@ __device__ __forceinline__ void flow_macros(const C* f, C& rho, C& jx, C& jy, C&
 template <int LAT, int i, class C>
 __device__ __forceinline__ C e_dot(C jx, C jy, C jz) {
   using L = Lattice<LAT>;
-  C v = C(0.);
+  C v = C(0);
   if constexpr (L::ex(i) == 1) v += jx;
   if constexpr (L::ex(i) == -1) v -= jx;
   if constexpr (L::ey(i) == 1) v += jy;

@@ -33,14 +33,40 @@
 // 0.14 to 0.40 forward, 0.19 to 0.69 reverse.
 #pragma once
 
+#include <type_traits>
+
 #include "lbm_device.cuh"
 
 namespace lbm {
 namespace fx {
 
-typedef long long i64;
 typedef unsigned long long u64;
 typedef unsigned int u32;
+
+// Two's-complement integers of 64 bits whose sums, differences, products and
+// shifts wrap.  The collision relies on it: the terms of a bounded result may
+// leave the range on the way (a product of a factor above 1/2 does, see mulc), which
+// a built-in signed type leaves undefined.
+struct i64 {
+  u64 v;
+  i64() = default;
+  template <class T, class = typename std::enable_if<std::is_integral<T>::value>::type>
+  __device__ __forceinline__ constexpr i64(T x) : v(static_cast<u64>(x)) {}
+  __device__ __forceinline__ explicit operator u64() const { return v; }
+  __device__ __forceinline__ explicit operator long long() const { return (long long)v; }
+  __device__ __forceinline__ explicit operator int() const { return (int)(u32)v; }
+  __device__ __forceinline__ friend i64 operator+(i64 a, i64 b) { return i64(a.v + b.v); }
+  __device__ __forceinline__ friend i64 operator-(i64 a, i64 b) { return i64(a.v - b.v); }
+  __device__ __forceinline__ friend i64 operator*(i64 a, i64 b) { return i64(a.v * b.v); }
+  __device__ __forceinline__ friend i64 operator^(i64 a, i64 b) { return i64(a.v ^ b.v); }
+  __device__ __forceinline__ friend i64 operator&(i64 a, i64 b) { return i64(a.v & b.v); }
+  __device__ __forceinline__ i64 operator-() const { return i64(0ull - v); }
+  __device__ __forceinline__ i64 operator<<(int n) const { return i64(v << n); }
+  __device__ __forceinline__ i64 operator>>(int n) const { return i64((long long)v >> n); }
+  __device__ __forceinline__ i64& operator+=(i64 b) { return *this = *this + b; }
+  __device__ __forceinline__ i64& operator-=(i64 b) { return *this = *this - b; }
+  __device__ __forceinline__ bool negative() const { return (long long)v < 0; }
+};
 
 constexpr int kScale = 61;   // populations, moments and increments: value * 2^61
 
@@ -76,9 +102,9 @@ __device__ __forceinline__ double from_words(u32 hi, u32 lo) {
 }
 __device__ __forceinline__ double from_int(i64 v) {
 #if defined(__CUDA_ARCH__)
-  return __ll2double_rn(v);
+  return __ll2double_rn((long long)v);
 #else
-  return (double)v;
+  return (double)(long long)v;
 #endif
 }
 
@@ -108,7 +134,7 @@ __device__ __forceinline__ double to_double(i64 v, int k) {
 // operators: up to 21 such cells without it, none with it.
 __device__ __forceinline__ i64 apart(i64 v) {
 #if defined(__CUDA_ARCH__)
-  asm("" : "+l"(v));
+  asm("" : "+l"(v.v));
 #endif
   return v;
 }
@@ -882,7 +908,7 @@ struct Stress2 {
 };
 
 __device__ __forceinline__ u128 square(i64 a) {
-  const u64 m = (u64)(a < 0 ? -a : a);
+  const u64 m = (u64)(a.negative() ? -a : a);
   return (u128)m * m;
 }
 // a * c / 2^64
