@@ -128,10 +128,13 @@ __device__ __forceinline__ double to_double(i64 v, int k) {
 
 // A product kept apart from the sums it enters.  Without this the compiler
 // gathers the subtracted halves of several signed products into one sum and
-// drops the carry of its subtraction where the sum's low word is zero: one reverse
-// step in about 2^31 came out wrong by 2^32 units (4e-8 of a population of the
-// cell).  Over 1e10 to 4e10 random cells per model and direction against the FP64
-// operators: up to 21 such cells without it, none with it.
+// drops the carry of its subtraction where the sum's low word is zero: 0 to 7
+// of some 4e9 random cells (per model; all of them reverse steps) came out
+// wrong by 2^32 units, 4e-8 of a population, and none of 1e10 to 4e10 with it.
+// States and adjoints whose words are zero show it at once: without apart,
+// 27 of the 36 cases of reverse steps in tests/test_gpu_fixed_words.py fail, over
+// all models; with it none does, nor do the sums that have no such product
+// (PairDot, the moments).
 __device__ __forceinline__ i64 apart(i64 v) {
 #if defined(__CUDA_ARCH__)
   asm("" : "+l"(v.v));
