@@ -57,7 +57,13 @@ extern "C" {
 /* Population storage in device memory.  Compute precision is FP64 for
  * LBM_STORE_FP64 (collisions of cells near equilibrium in 64-bit fixed point,
  * with a smaller error than the FP64 expressions) and FP32 for the two shifted
- * forms, which store the deviation f_i - w_i. */
+ * forms, which store the deviation f_i - w_i.
+ * With a velocity objective (THROUGH_FLOW, OUTFLOW, HEAT_FLUX) the steps t at
+ * which the flow from a fluid at rest has not reached the objective's cells run
+ * the FP64 expressions, which are several times slower: t < 1.1 sqrt(3) d + 30, d
+ * the distance in cells from the nearest boundary that drives the flow, and every
+ * t where none does.  It depends on the model and on t alone, not on the state,
+ * on how a sweep is cut into calls or on earlier calls. */
 #define LBM_STORE_FP64 0
 #define LBM_STORE_FP32 1
 #define LBM_STORE_FP16 2
@@ -344,16 +350,17 @@ int lbm_gradient_steady(lbm_handle* h, int max_steady, int check_every, double t
  * (which = 0), reverse steps over the current state (which = 1; the forward
  * state is left unchanged) or forward+reverse pairs (which = 2) on the
  * handle's stream, bracketed by CUDA events recorded on that stream.  *ms
- * gets the elapsed time.  The adjoint and sensitivity fields are scratch
- * afterwards. */
+ * gets the elapsed time.  Each step runs the operators of its own time (see
+ * LBM_STORE_FP64).  The adjoint and sensitivity fields are scratch afterwards. */
 int lbm_time_steps(lbm_handle* h, int which, int nsteps, float* ms);
 
 /* Time every candidate thread-block shape of the forward and reverse step
  * kernels (and both register variants of the reverse step) for nsteps steps
  * each on this handle's lattice and keep the fastest (the tile-shape
  * autotuner).  Forward steps are timed with the objective summed over the
- * steps, as a gradient's forward sweep runs them.  Needs a design and a state; the state
- * is left unchanged and the adjoint and sensitivity fields are zeroed. */
+ * steps, as a gradient's forward sweep runs them, with the operators of its later steps
+ * (see LBM_STORE_FP64).  Needs a design and a state; the state is left unchanged and the
+ * adjoint and sensitivity fields are zeroed. */
 int lbm_autotune(lbm_handle* h, int nsteps);
 
 /* Block shape in use for the forward (which = 0) or reverse (which = 1) step. */

@@ -31,10 +31,6 @@ inline unsigned long long fixed_constant(long double v, int bits, bool& ok) {
 inline FixedModel fixed_model(const lbm_config& c) {
   FixedModel m = {};
   if (c.storage != LBM_STORE_FP64) return m;
-  // lattices too small for a velocity objective to stand clear of rounding
-  // (12 cells to average over on 36x36, MRT step 7.4 against 3.4 us)
-  const int64_t ncell = (int64_t)c.nx * c.ny * (c.lattice == LBM_D3Q19 ? c.nz : 1);
-  if (velocity_objective(c) && ncell < 2048) return m;
   bool ok = true;
   const long double om = c.omega;
   if (c.lattice == LBM_D3Q19 && c.collision == LBM_MRT) {
@@ -76,18 +72,19 @@ inline FixedModel fixed_model(const lbm_config& c) {
   return m;
 }
 
-// A velocity objective of a flow that is still at rest is nothing but rounding:
-// sweeps too short for the flow to reach the objective's cells keep the FP64
-// operators, whose rounding is the reference's.
-//
-// Steps after which a velocity objective measures a flow and no longer the
-// rounding of one at rest: one and a half times what sound (1/sqrt(3) cells a
-// step) takes from the nearest boundary that drives the flow to the cells that
-// the objective averages over, and 100.  (A heat flux sums over its box, where
-// only the warm part counts: to the middle.)  On the 201x201 pump the
-// pressure wave takes 164 steps to the outlets; its objective is 3e-10 after
-// 150 steps and 1e-6 after 250.  INT_MAX where no boundary drives the flow.
-// 0 for the other objectives.
+// Steps t whose state f_t keeps the FP64 operators, forward and reverse: a
+// velocity objective of a flow that is still at rest is nothing but rounding, and
+// the FP64 operators' rounding is the reference's.  The rule is one of the model
+// and of t alone, so that a sweep gives the same bits however it is cut into
+// calls.  1.1 times what sound (1/sqrt(3) cells a step) takes from the nearest
+// boundary that drives the flow to the cells that the objective averages over, and
+// 30 for the front to rise.  (A heat flux sums over its box, where only the warm
+// part counts: to the middle.)  By then the objective, summed with a weight of
+// one, is above 1e-7 on pumps of 60x60 to 420x420 cells and above 1e-6 soon
+// after, where the roundings of one step add 3e-16 (201x201 MRT: sound takes 164
+// steps; 1e-15 after 115, 1e-7 after 153, 1e-5 after 199; kept to 211).
+// Later steps cost 4.3 / 6.3 us (201x201, forward / reverse), these 21 / 49.
+// INT_MAX where no boundary drives the flow, 0 for the other objectives.
 inline int flow_start_up(const lbm_config& c) {
   ObjectiveInfo oi;
   if (!velocity_objective(c) || !objective_info(c.objective, &oi)) return 0;
@@ -116,7 +113,7 @@ inline int flow_start_up(const lbm_config& c) {
       if (best < 0. || d2 < best) best = d2;
     }
   }
-  return best < 0. ? INT_MAX : (int)(1.5 * sqrt(3. * best)) + 100;
+  return best < 0. ? INT_MAX : (int)(1.1 * sqrt(3. * best)) + 30;
 }
 
 }  // namespace lbm

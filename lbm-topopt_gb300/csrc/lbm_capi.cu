@@ -224,8 +224,8 @@ struct lbm_handle {
   void* lam[2] = {nullptr, nullptr};
   int lcur = 0;
   FixedModel fix = {};                 // fixed-point form of the FP64 collision
-  int start_up = 0;                    // steps until the objective sees the flow (flow_start_up)
-  int horizon = 0;                     // last step of the sweep being taken
+  int start_up = 0;                    // steps that keep the FP64 operators (flow_start_up)
+  bool past_start_up = false;          // all steps as later ones (while a tuner times them)
   unsigned long long* im = nullptr;    // its porosity planes (KParams::im, dimult)
   double* dimult = nullptr;
   unsigned long long* om6 = nullptr;   // and the thermal lattice's (om6, domega)
@@ -596,7 +596,7 @@ KParams base_params(const lbm_handle* h, int t) {
   p.sens = h->sens;
   p.sens_atomic = h->sens_atomic ? 1 : 0;
   p.fix = h->fix;
-  if (h->horizon < h->start_up) p.fix.ok = 0;
+  if (t < h->start_up && !h->past_start_up) p.fix.ok = 0;
   p.im = h->im;
   p.dimult = h->dimult;
   p.om6 = h->om6;
@@ -629,10 +629,17 @@ int launch(lbm_handle* h, int kind, const KParams& p, double* aux) {
   return 0;
 }
 
-// The step that n more steps lead to.
-int end_step(const lbm_handle* h, int64_t n) {
-  return (int)std::min<int64_t>((int64_t)h->t + n, INT_MAX - 1);
-}
+// Steps of the handles timed with the operators of a developed flow, as a
+// sweep's later ones run, while it lives.
+struct PastStartUp {
+  lbm_handle* const* h;
+  int n;
+  PastStartUp(lbm_handle* const* handles, int count) : h(handles), n(count) { set(true); }
+  ~PastStartUp() { set(false); }
+  void set(bool on) {
+    for (int i = 0; i < n; ++i) h[i]->past_start_up = on;
+  }
+};
 
 int ensure_jcap(lbm_handle* h, size_t n) {
   if (n <= h->jcap) return 0;
@@ -939,6 +946,7 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   ALLOC(h->lam[1], adjoint_bytes(h));
   h->fix = fixed_model(c);
   h->start_up = flow_start_up(c);
+  if (h->start_up == INT_MAX) h->fix.ok = 0;   // no step would use it
   // the design's planes: gamma and, of 8 bytes a cell as well (FP64 storage),
   // those of the fixed-point collisions
   const int planes = !h->fix.ok ? 1 : c.lattice == LBM_D2Q9_D2Q5 ? 5 : 3;
@@ -1152,7 +1160,6 @@ int lbm_forward_steady(lbm_handle* h, int max_steps, int check_every, double tol
   if (!h->have_state) return fail(h, LBM_ERR_STATE, "no state (lbm_init_equilibrium)");
   int rc = ensure_jcap(h, 1);
   if (rc) return rc;
-  h->horizon = end_step(h, max_steps);
   unsigned long long* bits = (unsigned long long*)h->jdev;
   double last = -1.;
   int k = 0;
@@ -1248,7 +1255,6 @@ int lbm_forward(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
   if (nsteps == 0) return LBM_OK;
   const bool obj = h->cfg.objective != LBM_OBJ_NONE;
   int rc;
-  h->horizon = end_step(h, nsteps);
   if (!obj) {
     for (int k = 0; k < nsteps; ++k)
       if ((rc = forward_step(h, nullptr))) return rc;
@@ -1347,7 +1353,6 @@ int lbm_adjoint_step(lbm_handle* h) {
   if (!h->have_design || !h->have_state) return fail(h, LBM_ERR_STATE, "no design or state");
   if (!h->have_adjoint) return fail(h, LBM_ERR_STATE, "adjoint not reset (lbm_adjoint_reset)");
   int rc;
-  h->horizon = std::max(h->horizon, h->t);
   if (h->cfg.objective == LBM_OBJ_REGENERATOR_EFFICIENCY && h->t >= h->obj_from) {
     // this step's share of the 1/D design term needs the step's objective
     if ((rc = ensure_jcap(h, 1))) return rc;
@@ -1463,8 +1468,6 @@ int gradient_run(lbm_handle* h, int nsteps, int nsnap, int schedule, SteadyPhase
 
   h->t_phase = INT_MAX;   // a new run: ramps wait for the steady phase
   h->obj_from = 1;
-  h->t = 0;
-  h->horizon = end_step(h, sp ? (int64_t)sp->max_steps + nsteps : nsteps);
   cudaEventRecord(h->ev[0], h->stream);
   {
     const int out = pool.scratch();
@@ -1593,8 +1596,6 @@ int lbm_time_steps(lbm_handle* h, int which, int nsteps, float* ms) {
     h->have_adjoint = true;
   }
   int t_keep = h->t;
-  const int horizon_keep = h->horizon;
-  h->horizon = INT_MAX;   // as in a long sweep
   if (which == 1 && h->t < 1) h->t = 1;
   cudaEventRecord(h->ev[0], h->stream);
   for (int k = 0; k < nsteps; ++k) {
@@ -1606,10 +1607,8 @@ int lbm_time_steps(lbm_handle* h, int which, int nsteps, float* ms) {
       rc = forward_step(h, nullptr);
       if (!rc) rc = adjoint_step(h);
     }
-    if (rc) break;
+    if (rc) return rc;
   }
-  h->horizon = horizon_keep;
-  if (rc) return rc;
   cudaEventRecord(h->ev[1], h->stream);
   if ((rc = sync(h))) return rc;
   if (which == 1) h->t = t_keep;
@@ -1626,8 +1625,8 @@ int lbm_autotune(lbm_handle* h, int nsteps) {
   void* keep = nullptr;
   CUDA_OR_FAIL(h, cudaMalloc(&keep, state_bytes(h)));
   CUDA_OR_FAIL(h, cudaMemcpyAsync(keep, h->f[h->cur], state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
-  const int t_keep = h->t, cur_keep = h->cur, horizon_keep = h->horizon;
-  h->horizon = INT_MAX;   // as in a long sweep
+  const int t_keep = h->t, cur_keep = h->cur;
+  const PastStartUp developed(&h, 1);
   if (!h->have_adjoint) {
     if ((rc = zero_adjoint(h))) { cudaFree(keep); return rc; }
     h->have_adjoint = true;
@@ -1672,7 +1671,6 @@ int lbm_autotune(lbm_handle* h, int nsteps) {
   h->tuned = true;
   h->cur = cur_keep;
   h->t = t_keep;
-  h->horizon = horizon_keep;
   CUDA_OR_FAIL(h, cudaMemcpyAsync(h->f[h->cur], keep, state_bytes(h), cudaMemcpyDeviceToDevice, h->stream));
   rc = zero_adjoint(h);
   if (!rc) rc = sync(h);
@@ -2032,8 +2030,6 @@ int batch_sequence(lbm_batch* b, int nsteps, int nsnap, int schedule, int64_t* r
   for (int i = 0; i < b->n; ++i) {
     b->h[i]->cur = 0;
     b->h[i]->lcur = 0;
-    b->h[i]->t = 0;
-    b->h[i]->horizon = nsteps;
   }
   WangSchedule ws(nsnap);
   const bool planned = schedule == LBM_SCHEDULE_STATIC;
@@ -2223,8 +2219,8 @@ int lbm_batch_autotune(lbm_batch* b, int nsteps) {
     for (void* p : h->lam) BCUDA(b, cudaMemsetAsync(p, 0, adjoint_bytes(h), b->stream));
     h->have_adjoint = true;
     h->t = 1;
-    h->horizon = INT_MAX;   // as in a long sweep
   }
+  const PastStartUp developed(b->h, b->n);
   // each kernel on its own: every shape for the forward step, then every
   // shape and both register variants for the reverse step
   float best_f = 1e30f, best_a = 1e30f;
@@ -2357,7 +2353,6 @@ int lbm_batch_forward(lbm_batch* b, int nsteps, double* J) {
   double* res[LBM_MAX_BATCH];
   for (int i = 0; i < b->n; ++i) {
     res[i] = b->h[i]->jdev;
-    b->h[i]->horizon = end_step(b->h[i], nsteps);
   }
   for (int i = 0; i < b->n && !rc; ++i)
     if (b->h[i]->cfg.objective != LBM_OBJ_NONE && (rc = begin_accumulate(b->h[i], b->stream)))
@@ -2505,7 +2500,6 @@ int lbm_batch_time_steps(lbm_batch* b, int which, int nsteps, float* ms) {
       h->have_adjoint = true;
     }
     if (which >= 1 && h->t < 1) h->t = 1;
-    h->horizon = INT_MAX;   // as in a long sweep
   }
   cudaEventRecord(b->ev[0], b->stream);
   for (int k = 0; k < nsteps; ++k) {
