@@ -18,9 +18,9 @@
 #include "../../include/lbmgpu.h"
 #include "fixed_model.hpp"
 #include "host_buffers.hpp"
-#include "mapped_slots.hpp"
 #include "lbm_device.cuh"
 #include "lbm_ops.h"
+#include "mapped_result.hpp"
 #include "state_pool.hpp"
 #include "wang.hpp"
 
@@ -235,8 +235,7 @@ struct lbm_handle {
   unsigned* counter = nullptr;
   double* jdev = nullptr;
   size_t jcap = 0;
-  double* jhost = nullptr;       // a result and a flag in mapped host memory, and their
-  double* jhost_dev = nullptr;   // device address
+  MappedResult jmap;             // a result and a flag in mapped host memory
   double* step_partial = nullptr;   // warp partials of kept steps (lbm_forward's J_steps)
   int step_rows = 0;                // steps it holds
   double* step_row = nullptr;       // the row the next objective adds into (null: `partial`)
@@ -501,8 +500,7 @@ void destroy_buffers(lbm_handle* h) {
   h->om6 = nullptr;
   h->counter = nullptr;
   h->jdev = h->stage = h->init_mac = h->step_partial = nullptr;
-  if (h->jhost) MappedSlots::give(h->jhost);   // the stream's work is done
-  h->jhost = h->jhost_dev = nullptr;
+  h->jmap.give();   // the stream's work is done
   for (cudaEvent_t& e : h->ev)
     if (e) {
       cudaEventDestroy(e);
@@ -653,15 +651,6 @@ int ensure_jcap(lbm_handle* h, size_t n) {
 
 // Design values from which on the range check runs on the device.
 constexpr int64_t kDeviceCheck = 8192;
-
-int ensure_jhost(lbm_handle* h) {
-  if (h->jhost) return 0;
-  cudaError_t e = cudaSuccess;
-  h->jhost = (double*)MappedSlots::take(&e);
-  CUDA_OR_FAIL(h, e);
-  CUDA_OR_FAIL(h, cudaHostGetDevicePointer((void**)&h->jhost_dev, h->jhost, 0));
-  return 0;
-}
 
 // Rows for the objectives of up to 64 single steps, within 32 MB.
 int ensure_step_rows(lbm_handle* h) {
@@ -1087,10 +1076,10 @@ int lbm_set_design(lbm_handle* h, const double* gamma) {
   CUDA_OR_FAIL(h, cudaMemcpyAsync(h->stage, gamma, (size_t)h->ncell * sizeof(double),
                                   cudaMemcpyHostToDevice, h->stream));
   if (on_device) {
-    if ((rc = ensure_jhost(h))) return rc;
-    volatile int* bad = (volatile int*)(h->jhost + 1);
+    CUDA_OR_FAIL(h, h->jmap.take());
+    volatile int* bad = (volatile int*)(h->jmap.host + 1);
     *bad = 0;
-    k_check_unit<<<608, 256, 0, h->stream>>>(h->stage, (long long)h->ncell, (int*)(h->jhost_dev + 1));
+    k_check_unit<<<608, 256, 0, h->stream>>>(h->stage, (long long)h->ncell, (int*)(h->jmap.dev + 1));
     h->launches++;
     CUDA_OR_FAIL(h, cudaGetLastError());
     if ((rc = sync(h))) return rc;
@@ -1263,21 +1252,21 @@ int lbm_forward(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
     return LBM_OK;
   }
   if (J_steps) return forward_per_step(h, nsteps, J_steps, J_sum);
-  if ((rc = ensure_jhost(h))) return rc;
+  CUDA_OR_FAIL(h, h->jmap.take());
   if (nsteps == 1 && h->geo.nblocks <= kDirectBlocks) {
     // one state's objective: the objective kernel reduces it by itself
     if ((rc = forward_step(h, nullptr))) return rc;
-    if ((rc = objective_only(h, h->jhost_dev))) return rc;
+    if ((rc = objective_only(h, h->jmap.dev))) return rc;
   } else {
     if ((rc = begin_accumulate(h))) return rc;
-    for (int k = 0; k < nsteps && !rc; ++k) rc = forward_step(h, k > 0 ? h->jhost_dev : nullptr);
-    if (!rc) rc = objective_only(h, h->jhost_dev);
-    if (!rc) rc = end_accumulate(h, h->jhost_dev);
+    for (int k = 0; k < nsteps && !rc; ++k) rc = forward_step(h, k > 0 ? h->jmap.dev : nullptr);
+    if (!rc) rc = objective_only(h, h->jmap.dev);
+    if (!rc) rc = end_accumulate(h, h->jmap.dev);
     h->accumulate = false;
     if (rc) return rc;
   }
   if ((rc = sync(h))) return rc;
-  const double acc = *h->jhost;
+  const double acc = *h->jmap.host;
   if (!std::isfinite(acc)) return fail(h, LBM_ERR_NONFINITE, "objective is not finite");
   if (J_sum) *J_sum = acc;
   return LBM_OK;
