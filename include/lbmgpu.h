@@ -380,7 +380,10 @@ int lbm_set_launch_shape(lbm_handle* h, int which, int bx, int by);
  * 9e-10 of max |dJ/dgamma| on a D2Q9 channel; bit-identical on D3Q19 MRT and
  * the thermal model).  Set the variant explicitly for bitwise reproducible
  * FP32 gradients across tuning runs.  FP64 storage has only variant 0 (1
- * returns LBM_ERR_SUP).  No reference counterpart. */
+ * returns LBM_ERR_SUP); on D2Q9 its register budget follows the number of cells
+ * (one more resident block past 512 cells per SM) or lbm_autotune, with the same
+ * results, and setting 0 returns to the number of cells.  No reference
+ * counterpart. */
 int lbm_set_reverse_variant(lbm_handle* h, int lean);
 /* The reverse step variant in use (0 or 1), negative on error. */
 int lbm_get_reverse_variant(const lbm_handle* h);

@@ -212,8 +212,7 @@ struct lbm_handle {
   Geometry geo;       // initialisation / export kernels
   Geometry geo_fwd;   // forward step (autotuned)
   Geometry geo_adj;   // reverse step (autotuned)
-  bool adj_lean = false;   // reverse step: the register-lean variant (autotuned)
-  bool adj_wide = false;   // FP64 D2Q9 reverse step with three resident blocks (wide_reverse)
+  bool adj_lean = false;   // reverse step: the register-lean variant (wide_reverse, autotuned)
   bool sens_atomic = false;   // reverse step adds to dJ/dgamma atomically (fits in L2)
   bool tuned = false;
   int nsm = 1;
@@ -343,9 +342,9 @@ bool fits_in_l2(size_t bytes) {
   return bytes <= (size_t)l2;
 }
 
-// Whether the reverse steps of a lattice (or batch) of that many cells run with
-// one more resident block per SM by default: FP64 D2Q9 lattices past one wave
-// of two 256-thread blocks per SM (see Occupancy in lbm_kernels.cuh).
+// Whether the reverse steps of a lattice (or batch) of that many cells run the
+// register-lean variant by default: FP64 D2Q9 lattices past one wave of two
+// 256-thread blocks per SM (see Occupancy in lbm_kernels.cuh).
 bool wide_reverse(const lbm_config& c, int64_t ncell) {
   int dev = 0, nsm = 0;
   if (c.storage != LBM_STORE_FP64 || c.lattice != LBM_D2Q9) return false;
@@ -353,6 +352,11 @@ bool wide_reverse(const lbm_config& c, int64_t ncell) {
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return false;
   return ncell > (int64_t)nsm * 512;
+}
+
+// Whether the reverse step is built for two register budgets.
+bool two_reverse_budgets(const lbm_config& c) {
+  return c.storage != LBM_STORE_FP64 || c.lattice == LBM_D2Q9;
 }
 
 int check_box(const lbm_config& c, const int* b, int dim, const char* what) {
@@ -728,7 +732,7 @@ int adjoint_at(lbm_handle* h, const void* f) {
   p.lam_in = h->lam[h->lcur];
   p.lam_out = h->lam[1 - h->lcur];
   p.eval_obj = (h->t >= h->obj_from && h->cfg.objective != LBM_OBJ_NONE) ? 1 : 0;
-  int rc = launch(h, h->adj_lean || (h->adj_wide && p.fix.ok) ? K_ADJOINT_LEAN : K_ADJOINT, p, nullptr);
+  int rc = launch(h, h->adj_lean ? K_ADJOINT_LEAN : K_ADJOINT, p, nullptr);
   if (rc) return rc;
   h->lcur ^= 1;
   return 0;
@@ -876,7 +880,7 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   h->adj_bytes = c.storage == LBM_STORE_FP64 ? 8 : 4;
   h->gam_bytes = c.storage == LBM_STORE_FP64 ? 8 : 4;
   h->sens_atomic = fits_in_l2(reverse_step_bytes(h));
-  h->adj_wide = wide_reverse(c, h->ncell);
+  h->adj_lean = wide_reverse(c, h->ncell);
   h->launch = c.lattice == LBM_D2Q9    ? launcher_d2q9(c.collision, c.storage)
               : c.lattice == LBM_D3Q19 ? launcher_d3q19(c.collision, c.storage)
                                        : launcher_thermal(c.collision, c.storage);
@@ -1625,7 +1629,7 @@ int lbm_autotune(lbm_handle* h, int nsteps) {
   Geometry bf = h->geo_fwd, ba = h->geo_adj;
   bool blean = h->adj_lean;
   const int nx = h->cfg.nx;
-  const int nlean = h->cfg.storage == LBM_STORE_FP64 ? 1 : 2;   // FP64 has no lean variant
+  const int nlean = two_reverse_budgets(h->cfg) ? 2 : 1;
   // Forward steps are timed as a gradient's forward sweep runs them, with the
   // objective summed into the warp partials (scratch here; the next sweep
   // zeroes them): the shapes differ most in that reduction.
@@ -1692,14 +1696,14 @@ int lbm_set_reverse_variant(lbm_handle* h, int lean) {
   if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
   if (lean != 0 && lean != 1) return fail(h, LBM_ERR_ARG, "variant %d is neither 0 nor 1", lean);
   if (lean && h->cfg.storage == LBM_STORE_FP64)
-    return fail(h, LBM_ERR_SUP, "FP64 storage has no register-lean reverse variant");
-  h->adj_lean = lean == 1;
+    return fail(h, LBM_ERR_SUP, "FP64 storage has no reverse variant to choose");
+  h->adj_lean = lean == 1 || wide_reverse(h->cfg, h->ncell);
   return LBM_OK;
 }
 
 int lbm_get_reverse_variant(const lbm_handle* h) {
   if (!h) return fail(nullptr, LBM_ERR_ARG, "null handle");
-  return h->adj_lean ? 1 : 0;
+  return h->adj_lean && h->cfg.storage != LBM_STORE_FP64 ? 1 : 0;
 }
 
 int lbm_select_device(int ordinal) {
@@ -1796,8 +1800,7 @@ struct lbm_batch {
   cudaStream_t stream = nullptr;
   int bx = 128, by = 2;     // block shape of the forward and objective kernels
   int abx = 128, aby = 2;   // block shape of the reverse step kernel
-  bool adj_lean = false;    // reverse step: the register-lean variant
-  bool adj_wide = false;    // its default for FP64 D2Q9 (see lbm_handle)
+  bool adj_lean = false;    // reverse step: the register-lean variant (see lbm_handle)
   bool sens_atomic = false; // the batched reverse step fits in L2 (see lbm_handle)
   int nsm = 1;
   int grid_fwd = 1, grid_adj = 1, grid_obj = 1, grid_copy = 1;
@@ -1884,6 +1887,12 @@ void batch_layout(lbm_batch* b, BatchParams& bp, int kind) {
   bp.early = past_one_wave(b->h[0]->cfg, (size_t)start * blk.x * blk.y, b->nsm);
 }
 
+int64_t batch_cells(const lbm_batch* b) {
+  int64_t n = 0;
+  for (int i = 0; i < b->n; ++i) n += b->h[i]->ncell;
+  return n;
+}
+
 // Persistent grids of the batched kernels for the current block shapes.
 void batch_set_grids(lbm_batch* b) {
   BatchParams bp;
@@ -1892,8 +1901,7 @@ void batch_set_grids(lbm_batch* b) {
   batch_layout(b, bp, K_OBJECTIVE);
   b->grid_obj = batch_grid(b, K_OBJECTIVE, bp.start[b->n]);
   batch_layout(b, bp, K_ADJOINT);
-  b->grid_adj =
-      batch_grid(b, b->adj_lean || b->adj_wide ? K_ADJOINT_LEAN : K_ADJOINT, bp.start[b->n]);
+  b->grid_adj = batch_grid(b, b->adj_lean ? K_ADJOINT_LEAN : K_ADJOINT, bp.start[b->n]);
 }
 
 int batch_launch(lbm_batch* b, int kind, const BatchParams& bp, int grid) {
@@ -1973,7 +1981,7 @@ int batch_adjoint(lbm_batch* b, int buf) {
     p.eval_obj = (h->t >= 1 && h->cfg.objective != LBM_OBJ_NONE) ? 1 : 0;
     p.sens_atomic = b->sens_atomic ? 1 : 0;
   }
-  int rc = batch_launch(b, b->adj_lean || b->adj_wide ? K_ADJOINT_LEAN : K_ADJOINT, bp, b->grid_adj);
+  int rc = batch_launch(b, b->adj_lean ? K_ADJOINT_LEAN : K_ADJOINT, bp, b->grid_adj);
   if (rc) return rc;
   for (int i = 0; i < b->n; ++i) b->h[i]->lcur ^= 1;
   return 0;
@@ -2164,12 +2172,8 @@ int lbm_batch_create(const lbm_config* cfgs, int n, lbm_batch** out) {
   batch_set_grids(b);
   b->grid_copy = 4 * b->nsm;
   size_t rev = 0;
-  int64_t cells = 0;
-  for (int i = 0; i < b->n; ++i) {
-    rev += reverse_step_bytes(b->h[i]);
-    cells += b->h[i]->ncell;
-  }
-  b->adj_wide = wide_reverse(cfgs[0], cells);
+  for (int i = 0; i < b->n; ++i) rev += reverse_step_bytes(b->h[i]);
+  b->adj_lean = wide_reverse(cfgs[0], batch_cells(b));
   b->sens_atomic = fits_in_l2(rev);
   *out = b;
   return LBM_OK;
@@ -2215,7 +2219,7 @@ int lbm_batch_autotune(lbm_batch* b, int nsteps) {
   float best_f = 1e30f, best_a = 1e30f;
   int fbx = b->bx, fby = b->by, abx = b->abx, aby = b->aby;
   bool alean = b->adj_lean;
-  const int nlean = b->h[0]->cfg.storage == LBM_STORE_FP64 ? 1 : 2;
+  const int nlean = two_reverse_budgets(b->h[0]->cfg) ? 2 : 1;
   // forward steps timed with the objectives summed into the warp partials, as
   // a gradient's forward sweep runs them (the partials are scratch here)
   double* res[LBM_MAX_BATCH] = {};
@@ -2298,9 +2302,9 @@ int lbm_batch_set_reverse_variant(lbm_batch* b, int lean) {
   if (!b) return bfail(nullptr, LBM_ERR_ARG, "null batch");
   if (lean != 0 && lean != 1) return bfail(b, LBM_ERR_ARG, "variant %d is neither 0 nor 1", lean);
   if (lean && b->h[0]->cfg.storage == LBM_STORE_FP64)
-    return bfail(b, LBM_ERR_SUP, "FP64 storage has no register-lean reverse variant");
+    return bfail(b, LBM_ERR_SUP, "FP64 storage has no reverse variant to choose");
   batch_destroy_graph(b);
-  b->adj_lean = lean == 1;
+  b->adj_lean = lean == 1 || wide_reverse(b->h[0]->cfg, batch_cells(b));
   batch_set_grids(b);
   return LBM_OK;
 }
@@ -2326,7 +2330,7 @@ int lbm_batch_set_launch_shape(lbm_batch* b, int which, int bx, int by) {
 
 int lbm_batch_get_reverse_variant(const lbm_batch* b) {
   if (!b) return bfail(nullptr, LBM_ERR_ARG, "null batch");
-  return b->adj_lean ? 1 : 0;
+  return b->adj_lean && b->h[0]->cfg.storage != LBM_STORE_FP64 ? 1 : 0;
 }
 
 int lbm_batch_forward(lbm_batch* b, int nsteps, double* J) {
