@@ -149,11 +149,16 @@ Geometry row_blocks(const lbm_config& c, int nz, int threads) {
   return make_geometry(c.nx, c.ny, nz, bx, threads / bx);
 }
 
-// Whether that many threads are more than the forward step keeps resident at
-// once (Occupancy in lbm_kernels.cuh).
-bool past_one_wave(const lbm_config& c, size_t threads, int nsm) {
-  const int blocks = c.storage == LBM_STORE_FP64 ? 2 : c.lattice == LBM_D2Q9 ? 6 : 5;
-  return threads > (size_t)nsm * blocks * 256;
+// Whether a grid of that many threads lets the next launch proceed early
+// (step_prologue, which asks FP32 and FP16 kernels only): more of them than the
+// forward step keeps resident at once (Occupancy in lbm_kernels.cuh).  The
+// reverse step keeps fewer, but its line lies at the same number: with a line of
+// its own (4 blocks of 256 per SM, 3 for D3Q19 BGK) grids between the two take, in
+// us a reverse step, FP32 512x384 5.36 against 5.67, thermal 512x320 7.20 / 7.36,
+// duct 64x48x54 8.15 / 8.34, FP16 512x384 5.53 / 5.79, and as parts of
+// forward and reverse pairs 0 to 11% more; only FP16 ducts gain, by 1 to 3%.
+bool starts_early(const lbm_config& c, size_t threads, int nsm) {
+  return threads > (size_t)nsm * (c.lattice == LBM_D2Q9 ? 6 : 5) * 256;
 }
 
 // Block shape of the step kernels of a handle that is not tuned, by the number
@@ -330,9 +335,11 @@ __global__ void k_box_add_scaled(double* __restrict__ sens, int nx, int ny, int 
 size_t state_bytes(const lbm_handle* h) { return (size_t)h->Q * h->P * h->pop_bytes; }
 size_t adjoint_bytes(const lbm_handle* h) { return (size_t)h->Q * h->P * h->adj_bytes; }
 // Bytes one reverse step moves: the state, the adjoint in and out, the design
-// and the FP64 dJ/dgamma read and written.
+// (or the planes of the fixed-point collision, of 8 bytes a cell) and the FP64
+// dJ/dgamma read and written.
 size_t reverse_step_bytes(const lbm_handle* h) {
-  return state_bytes(h) + 2 * adjoint_bytes(h) + (size_t)h->P * (h->gam_bytes + 16);
+  const size_t design = !h->fix.ok ? h->gam_bytes : h->cfg.lattice == LBM_D2Q9_D2Q5 ? 32 : 16;
+  return state_bytes(h) + 2 * adjoint_bytes(h) + (size_t)h->P * (design + 16);
 }
 // Whether a reverse step of that many bytes stays in this device's L2.
 bool fits_in_l2(size_t bytes) {
@@ -525,8 +532,8 @@ KParams base_params(const lbm_handle* h, int t) {
   p.step = (unsigned)t;
   p.key_fwd = step_key(p.step, kSaltForward);
   p.key_adj = step_key(p.step, kSaltAdjoint);
-  p.early_fwd = past_one_wave(c, h->geo_fwd.threads(), h->nsm);
-  p.early_adj = past_one_wave(c, h->geo_adj.threads(), h->nsm);
+  p.early_fwd = starts_early(c, h->geo_fwd.threads(), h->nsm);
+  p.early_adj = starts_early(c, h->geo_adj.threads(), h->nsm);
   p.omega = c.omega;
   for (int i = 0; i < 8; ++i) p.mrt[i] = c.mrt[i];
   p.pbb_scale = c.interp_scale;
@@ -879,7 +886,6 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   h->pop_bytes = c.storage == LBM_STORE_FP64 ? 8 : c.storage == LBM_STORE_FP32 ? 4 : 2;
   h->adj_bytes = c.storage == LBM_STORE_FP64 ? 8 : 4;
   h->gam_bytes = c.storage == LBM_STORE_FP64 ? 8 : 4;
-  h->sens_atomic = fits_in_l2(reverse_step_bytes(h));
   h->adj_lean = wide_reverse(c, h->ncell);
   h->launch = c.lattice == LBM_D2Q9    ? launcher_d2q9(c.collision, c.storage)
               : c.lattice == LBM_D3Q19 ? launcher_d3q19(c.collision, c.storage)
@@ -940,6 +946,7 @@ int lbm_create(const lbm_config* cfg, lbm_handle** out) {
   h->fix = fixed_model(c);
   h->start_up = flow_start_up(c);
   if (h->start_up == INT_MAX) h->fix.ok = 0;   // no step would use it
+  h->sens_atomic = fits_in_l2(reverse_step_bytes(h));
   // the design's planes: gamma and, of 8 bytes a cell as well (FP64 storage),
   // those of the fixed-point collisions
   const int planes = !h->fix.ok ? 1 : c.lattice == LBM_D2Q9_D2Q5 ? 5 : 3;
@@ -1884,7 +1891,7 @@ void batch_layout(lbm_batch* b, BatchParams& bp, int kind) {
   // slots past the batch start at the total (the kernels count the starts
   // at or below a block)
   for (int i = b->n; i <= kMaxBatch; ++i) bp.start[i] = start;
-  bp.early = past_one_wave(b->h[0]->cfg, (size_t)start * blk.x * blk.y, b->nsm);
+  bp.early = starts_early(b->h[0]->cfg, (size_t)start * blk.x * blk.y, b->nsm);
 }
 
 int64_t batch_cells(const lbm_batch* b) {

@@ -268,7 +268,7 @@ struct KParams {
   long long P;       // plane stride in elements
   unsigned step;     // time step of the input state
   unsigned key_fwd, key_adj;   // rounding-stream keys of the two step kernels at this step
-  int early_fwd, early_adj;    // their grids are more than one wave (step_prologue)
+  int early_fwd, early_adj;    // whether they let the next launch proceed early (step_prologue)
   // model
   double omega;
   double mrt[8];
@@ -1996,7 +1996,7 @@ struct BatchParams {
   // multiply-high form does not apply (a divisor of 1, or a product n * d
   // that can reach 2^32)
   unsigned gxm[kMaxBatch], gym[kMaxBatch];
-  int early;                    // the grid is more than one wave (step_prologue)
+  int early;                    // whether it lets the next launch proceed early (step_prologue)
   KParams p[kMaxBatch];
 };
 
