@@ -56,8 +56,9 @@ extern "C" {
 
 /* Population storage in device memory.  Compute precision is FP64 for
  * LBM_STORE_FP64 (collisions of cells near equilibrium in 64-bit fixed point,
- * with a smaller error than the FP64 expressions) and FP32 for the two shifted
- * forms, which store the deviation f_i - w_i.
+ * whose error, root mean square over cells and relative to a cell's largest
+ * population or adjoint, is no larger than the FP64 expressions') and FP32 for
+ * the two shifted forms, which store the deviation f_i - w_i.
  * With a velocity objective (THROUGH_FLOW, OUTFLOW, HEAT_FLUX) the steps t at
  * which the flow from a fluid at rest has not reached the objective's cells run
  * the FP64 expressions, which are several times slower: t < 1.1 sqrt(3) d + 30, d
