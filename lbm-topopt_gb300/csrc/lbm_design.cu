@@ -385,7 +385,8 @@ __global__ void __launch_bounds__(kThreads) k_mma_gensub(MmaDev d, MmaScalars s,
     d.q0[i] = xl * xl * (fmax(0., -df) + 0.001 * fabs(df) + reg);
 #pragma unroll
     for (int j = 0; j < M; ++j) {
-      const double gj = d.dg[(long long)j * d.n + i];
+      double gj = d.dg[(long long)j * d.n + i];
+      if (gj != gj) gj = 0.;   // max(0, g) of what is not a number
       const double h = gj > 0. ? ux : xl;
       d.G[(long long)j * d.n + i] = h * h * gj;
       acc[j] += h * fabs(gj);
