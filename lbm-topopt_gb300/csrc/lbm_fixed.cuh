@@ -970,8 +970,8 @@ struct Dissipation2 {
   // The finest scale of a Block whose units take the source times the weight
   // (scaled): its error, some units of w 2^-61, is far above 2^-89 w.  Where the
   // adjoint is much smaller than the source (the first reverse steps, a fluid at
-  // rest) its own finer units would not: such cells took an FP64 sum until then,
-  // and a 2048x1024 reverse step whose flow had not developed 200 us, now 141.
+  // rest) its own finer units would not: with an FP64 sum for such cells a
+  // 2048x1024 reverse step whose flow has not developed takes 200 us against 141.
   __device__ __forceinline__ int scale_limit(const FixedModel& m) const {
     const i64 v[7] = {src.ev[0], src.ev[1], src.ev[2], src.ev[3], src.ev[4], src.gx, src.gy};
     u64 any = 1u;

@@ -333,10 +333,10 @@ struct FixedDesign {
 
 // Objective contribution of a thread's cells in a fixed-point step.  The
 // dissipation of the cells that run in fixed point, which every cell of the
-// lattice contributes, is kept as an integer and summed over the warp as one:
-// its conversions, products and the shuffle tree were 22 FP64 operations a cell,
-// 19 us of the 33 us forward step on the 1024x512 channel, which now takes
-// 23 us (14 us without an objective).
+// lattice contributes, is kept as an integer and summed over the warp as one: in
+// FP64 its conversions, products and the shuffle tree are 22 operations a cell,
+// and the forward step of the 1024x512 channel takes 33 us against 23 (14
+// without an objective).
 template <int LAT>
 struct FixedObjective {
   double v = 0.;
