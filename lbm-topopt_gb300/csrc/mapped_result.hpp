@@ -1,10 +1,12 @@
-// mapped_result.hpp -- a handle's small results in host memory that the GPU maps.
+// mapped_result.hpp -- a handle's small results in host memory that the GPU writes.
 //
 // A kernel writes an objective or a flag straight into host memory, without a
 // copy behind it.  Each handle has a page of its own, so nothing is shared
-// between handles or threads and nothing outlives the handle: 8 us to register
-// and 11 us to give back on the GB300 host, where cudaHostAlloc and cudaFreeHost
-// take 100 and 165.
+// between handles or threads and nothing outlives the handle.  GB300's GPU
+// reads the host's own page tables, so ordinary memory will do; elsewhere the
+// page is registered.  (On the GB300 host that takes 25 us, and giving it back
+// 20; cudaHostAlloc and cudaFreeHost take 100 and 165.  A single step of a 64x48
+// channel with its objective takes 24 us either way.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -20,6 +22,7 @@ struct MappedResult {
   static constexpr size_t kBytes = 64;
   double* host = nullptr;   // null until taken
   double* dev = nullptr;    // its device address
+  bool registered = false;
 
   // Takes the page, if there is none yet.  After an error there is none.
   cudaError_t take() {
@@ -29,10 +32,17 @@ struct MappedResult {
     void* p = nullptr;
     if (posix_memalign(&p, n, n) != 0) return cudaErrorMemoryAllocation;
     memset(p, 0, kBytes);
-    cudaError_t e = cudaHostRegister(p, kBytes, cudaHostRegisterMapped | cudaHostRegisterPortable);
-    void* d = nullptr;
-    if (e == cudaSuccess && (e = cudaHostGetDevicePointer(&d, p, 0)) != cudaSuccess)
-      cudaHostUnregister(p);
+    int device = 0, host_tables = 0;
+    void* d = p;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess)
+      e = cudaDeviceGetAttribute(&host_tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables,
+                                 device);
+    if (e == cudaSuccess && !host_tables) {
+      e = cudaHostRegister(p, kBytes, cudaHostRegisterMapped | cudaHostRegisterPortable);
+      if (e == cudaSuccess && (e = cudaHostGetDevicePointer(&d, p, 0)) != cudaSuccess)
+        cudaHostUnregister(p);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       free(p);
@@ -40,14 +50,16 @@ struct MappedResult {
     }
     host = (double*)p;
     dev = (double*)d;
+    registered = !host_tables;
     return cudaSuccess;
   }
   // Gives it back; the work that writes to it has ended.
   void give() {
     if (!host) return;
-    if (cudaHostUnregister(host) != cudaSuccess) cudaGetLastError();
+    if (registered && cudaHostUnregister(host) != cudaSuccess) cudaGetLastError();
     free(host);
     host = dev = nullptr;
+    registered = false;
   }
 };
 

@@ -6,7 +6,7 @@
 #include "mapped_result.hpp"
 
 static std::map<void*, int> registered;
-static int fail_register = 0, fail_pointer = 0, last_error = 0;
+static int fail_register = 0, fail_pointer = 0, fail_attribute = 0, host_tables = 0, last_error = 0;
 
 extern "C" {
 cudaError_t cudaHostRegister(void* p, size_t, unsigned) {
@@ -22,6 +22,16 @@ cudaError_t cudaHostUnregister(void* p) {
 cudaError_t cudaHostGetDevicePointer(void** d, void* p, unsigned) {
   if (fail_pointer || !registered.count(p)) return (cudaError_t)(last_error = cudaErrorInvalidValue);
   *d = p;
+  return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int* d) {
+  *d = 0;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+  if (fail_attribute || a != cudaDevAttrPageableMemoryAccessUsesHostPageTables)
+    return (cudaError_t)(last_error = cudaErrorInvalidValue);
+  *v = host_tables;
   return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {
@@ -49,6 +59,9 @@ int main() {
   fail_pointer = 1;
   CHECK(a.take() != cudaSuccess && !a.host && !a.dev && registered.empty() && last_error == 0);
   fail_pointer = 0;
+  fail_attribute = 1;
+  CHECK(a.take() != cudaSuccess && !a.host && !a.dev && registered.empty() && last_error == 0);
+  fail_attribute = 0;
   CHECK(a.take() == cudaSuccess && a.host && a.dev == a.host && registered.size() == 1);
   double* const first = a.host;
   CHECK(a.take() == cudaSuccess && a.host == first && registered.size() == 1);
@@ -66,6 +79,17 @@ int main() {
   CHECK(!a.host && last_error == 0);
   CHECK(a.take() == cudaSuccess && a.dev && registered.size() == 1);
   a.give();
+  // a GPU that reads the host's page tables takes the page as it is
+  host_tables = 1;
+  CHECK(a.take() == cudaSuccess && b.take() == cudaSuccess && registered.empty());
+  CHECK(a.host && a.dev == a.host && b.dev == b.host && a.host != b.host);
+  *a.host = 3.;
+  a.give();
+  host_tables = 0;
+  CHECK(a.take() == cudaSuccess && registered.size() == 1);
+  a.give();
+  b.give();
+  CHECK(!a.host && !b.host && registered.empty() && last_error == 0);
   printf("ok\n");
   return 0;
 }
