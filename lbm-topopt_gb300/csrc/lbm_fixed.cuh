@@ -346,6 +346,18 @@ __device__ __forceinline__ void mrt3d_collide(const i64* x, const Factor& im, co
 // of an FP64 sum over the cell; the derivative by imult takes the differences
 // as they are.
 
+// Whether all of v are finite and below 2^64: the transposed collision at such a state
+// takes an adjoint of zero to zero, in FP64 too.
+template <int N>
+__device__ __forceinline__ bool moderate(const double* v) {
+  u32 m = 0u;
+  static_for<N>([&](auto Q_) {
+    const u32 h = hi_word(v[decltype(Q_)::value]) & 0x7fffffffu;
+    m = h > m ? h : m;
+  });
+  return m < (1087u << 20);
+}
+
 template <int BITS>
 struct BlockOf {
   int k = 0;       // values * 2^k, the largest below 2^BITS

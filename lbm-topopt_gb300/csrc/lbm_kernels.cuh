@@ -531,7 +531,9 @@ __device__ __forceinline__ void adjoint_cell_fixed(const KParams& p, int x, int 
   }
   const bool diss =
       L::DIM == 2 && p.fix.ok && p.eval_obj && p.objective == LBM_OBJ_DISSIPATION;
-  // cells that no adjoint has reached yet keep their zeros
+  // cells that no adjoint has reached yet keep their zeros, unless their state has
+  // diverged: what is not a number shows
+  if (zero) zero = fx::moderate<L::Q>(f);
   if (!zero || diss) {
     fx::Window w;
     fx::i64 xi[L::QF];
