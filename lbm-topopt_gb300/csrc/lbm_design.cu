@@ -126,7 +126,14 @@ __global__ void k_gather_box(Grid g, const int* __restrict__ b, long long n,
 constexpr int kFilterX = 64, kFilterY = 4;
 __device__ __forceinline__ int rows(const Grid& g) { return g.ny * g.nz; }
 
-// Whether every tap of cell (x,y,z) stays within [lo, hi] of each axis.
+// Whether every tap of cell (x,y,z) stays within [lo, hi] of each axis.  The
+// kernels ask for all cells of a warp together (32 of one row): a warp that runs the
+// sum without tests for some cells and the one with them for the others takes longer
+// than with tests for all, and on fields of one wave the whole kernel with it
+// (physical() with radius 10 on 256x128: 83.5 us cell by cell, 68.6 so and with tests
+// for all; radius 8 on 1024x512: 281, 255 and 300).  Where no warp has its taps inside
+// (inner_warps) kernels without that sum run (INNER = false; radius 4 on 32x32x32:
+// 68.0 us with it, 58.0 without).
 __device__ __forceinline__ bool taps_inside(const StageDev& s, int x, int y, int z, int x0, int x1,
                                             int y0, int y1, int z0, int z1) {
   return x - s.reach >= x0 && x + s.reach <= x1 && y - s.reach >= y0 && y + s.reach <= y1 &&
@@ -134,9 +141,9 @@ __device__ __forceinline__ bool taps_inside(const StageDev& s, int x, int y, int
 }
 
 // acc + sum_k w_k v[offset_k], in tap order.  One FP64 multiply-add a tap bounds
-// the filters (two per clock and SM); with the bounds tests and three index
-// loads a tap that they ran with for every cell, the two stages (radii 8 and
-// 4) of a 1024x512 field took 350 us, against 210 us of multiply-adds.
+// the filters (two per clock and SM); with bounds tests and three index loads a tap
+// for every cell, the two stages (radii 8 and 4) of a 1024x512 field take 350 us,
+// against 210 us of multiply-adds.
 __device__ __forceinline__ double sum_taps(const StageDev& s, const double* __restrict__ v,
                                            double acc) {
   const long long* __restrict__ off = s.off;
@@ -146,22 +153,26 @@ __device__ __forceinline__ double sum_taps(const StageDev& s, const double* __re
   return acc;
 }
 
+template <bool INNER>
 __global__ void __launch_bounds__(kThreads) k_stage_forward(Grid g, StageDev s,
                                                             const double* __restrict__ in,
                                                             double* __restrict__ keep,
                                                             double* __restrict__ out) {
   const int x = blockIdx.x * kFilterX + threadIdx.x;
+  const unsigned live = __ballot_sync(0xffffffffu, x < g.nx);
   if (x >= g.nx) return;
   for (int r = blockIdx.y * kFilterY + threadIdx.y; r < rows(g); r += gridDim.y * kFilterY) {
     const int y = r % g.ny, z = r / g.ny;
     const long long c = ((long long)z * g.ny + y) * g.nx + x;
     const bool ib = in_box(s.box, x, y, z);
+    const bool inside = INNER && __all_sync(
+        live, !ib || taps_inside(s, x, y, z, 0, g.nx - 1, 0, g.ny - 1, 0, g.nz - 1));
     double v;
     if (!ib) {
       v = in[c];
     } else {
       double acc = 0.;
-      if (taps_inside(s, x, y, z, 0, g.nx - 1, 0, g.ny - 1, 0, g.nz - 1)) {
+      if (inside) {
         acc = sum_taps(s, in + c, acc);
       } else {
         for (int k = 0; k < s.ntaps; ++k) {
@@ -198,17 +209,19 @@ __global__ void __launch_bounds__(kThreads) k_stage_scale(Grid g, StageDev s,
 }
 
 // sout = H^T t: column c gathers the filter rows that hold it (the cone is symmetric)
+template <bool INNER>
 __global__ void __launch_bounds__(kThreads) k_stage_transpose(Grid g, StageDev s,
                                                               const double* __restrict__ t,
                                                               double* __restrict__ sout) {
   const int x = blockIdx.x * kFilterX + threadIdx.x;
+  const unsigned live = __ballot_sync(0xffffffffu, x < g.nx);
   if (x >= g.nx) return;
   const int* b = s.box;
   for (int r = blockIdx.y * kFilterY + threadIdx.y; r < rows(g); r += gridDim.y * kFilterY) {
     const int y = r % g.ny, z = r / g.ny;
     const long long c = ((long long)z * g.ny + y) * g.nx + x;
     double acc = in_box(b, x, y, z) ? 0. : t[c];
-    if (taps_inside(s, x, y, z, b[0], b[1], b[2], b[3], b[4], b[5])) {
+    if (INNER && __all_sync(live, taps_inside(s, x, y, z, b[0], b[1], b[2], b[3], b[4], b[5]))) {
       acc = sum_taps(s, t + c, acc);
     } else {
       for (int k = 0; k < s.ntaps; ++k) {
@@ -602,6 +615,14 @@ dim3 filter_grid(const Grid& g) {
 }
 const dim3 kFilterBlock(kFilterX, kFilterY);
 
+// Whether some warp of the filter kernels (32 cells from a multiple of 32 on) has all
+// its taps within x0..x1 of its row.
+bool inner_warps(const Grid& g, const StageDev& s, int x0, int x1) {
+  const int first = (x0 + s.reach + 31) / 32 * 32;
+  const int last = first + 31 < g.nx - 1 ? first + 31 : g.nx - 1;
+  return first <= last && last + s.reach <= x1;
+}
+
 int check_launch(lbm_topopt* t) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return tfail(t, LBM_ERR_CUDA, "kernel launch: %s", cudaGetErrorString(e));
@@ -619,8 +640,10 @@ int forward_chain(lbm_topopt* t, int r) {
   }
   for (int k = 0; k < t->nstages; ++k) {
     double* out = (k == t->nstages - 1) ? t->gamma[r] : t->tmp2;
-    k_stage_forward<<<filter_grid(t->g), kFilterBlock, 0, t->st>>>(t->g, stage_dev(t, k, r), in,
-                                                                   t->keep[r][k], out);
+    const StageDev s = stage_dev(t, k, r);
+    const auto kern = inner_warps(t->g, s, 0, t->g.nx - 1) ? k_stage_forward<true>
+                                                           : k_stage_forward<false>;
+    kern<<<filter_grid(t->g), kFilterBlock, 0, t->st>>>(t->g, s, in, t->keep[r][k], out);
     in = out;
   }
   return check_launch(t);
@@ -632,7 +655,9 @@ int transpose_chain(lbm_topopt* t, int r, double* out_design) {
   for (int k = t->nstages - 1; k >= 0; --k) {
     StageDev s = stage_dev(t, k, r);
     k_stage_scale<<<gb, kFilterBlock, 0, t->st>>>(t->g, s, t->keep[r][k], t->tmp, t->tmp2);
-    k_stage_transpose<<<gb, kFilterBlock, 0, t->st>>>(t->g, s, t->tmp2, t->tmp);
+    const auto kern = inner_warps(t->g, s, s.box[0], s.box[1]) ? k_stage_transpose<true>
+                                                               : k_stage_transpose<false>;
+    kern<<<gb, kFilterBlock, 0, t->st>>>(t->g, s, t->tmp2, t->tmp);
   }
   k_gather_box<<<grid_for(t->n), kThreads, 0, t->st>>>(t->g, t->box_d, t->n, t->tmp, out_design);
   return check_launch(t);
