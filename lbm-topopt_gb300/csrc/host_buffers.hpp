@@ -29,12 +29,6 @@ namespace lbm {
 // Where the kernel cannot, the copy makes them as it did before.
 inline void populate(void* p, size_t n) {
   if (!p || n < ((size_t)1 << 20)) return;
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
-  if (at.type != cudaMemoryTypeUnregistered) return;   // pinned, managed: pages are there
   const long ps = sysconf(_SC_PAGESIZE);
   if (ps <= 0) return;
   const uintptr_t page = (uintptr_t)ps, first = ((uintptr_t)p + page - 1) / page * page,
@@ -42,7 +36,7 @@ inline void populate(void* p, size_t n) {
   if (end <= first) return;
   const uintptr_t pages = (end - first) / page;
   int present = 0;
-  constexpr int kLook = 8;
+  constexpr int kLook = 3;
   for (int k = 0; k < kLook; ++k) {
     unsigned char in = 0;
     const uintptr_t at_page = first + (pages - 1) * k / (kLook - 1) * page;
@@ -50,6 +44,12 @@ inline void populate(void* p, size_t n) {
     present += in & 1;
   }
   if (present == kLook) return;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (at.type != cudaMemoryTypeUnregistered) return;   // pinned, managed: pages are there
   auto make = [=](uintptr_t from, uintptr_t to) {
     if (to > from) (void)madvise((void*)from, to - from, MADV_POPULATE_WRITE);
   };
