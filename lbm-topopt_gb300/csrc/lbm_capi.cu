@@ -239,7 +239,7 @@ struct lbm_handle {
   unsigned* counter = nullptr;
   double* jdev = nullptr;
   size_t jcap = 0;
-  MappedResult jmap;             // a result and a flag in mapped host memory
+  MappedResult jmap;             // small results in host memory: [0] a sum, [1] a flag, [4..7] steps
   double* step_partial = nullptr;   // warp partials of kept steps (lbm_forward's J_steps)
   int step_rows = 0;                // steps it holds
   double* step_row = nullptr;       // the row the next objective adds into (null: `partial`)
@@ -660,8 +660,8 @@ int ensure_jcap(lbm_handle* h, size_t n) {
   return 0;
 }
 
-// Design values from which on the range check runs on the device.
-constexpr int64_t kDeviceCheck = 8192;
+// Design values from which on the range check runs on the device (lbm_set_design).
+constexpr int64_t kDeviceCheck = 16384;
 
 // Rows for the objectives of up to 64 single steps, within 32 MB.
 int ensure_step_rows(lbm_handle* h) {
@@ -1078,8 +1078,8 @@ int lbm_set_design(lbm_handle* h, const double* gamma) {
   };
   // Large designs are checked on the device, before they replace the old one
   // (the loop above takes 1 ns a value: 4.2 ms for 256x128x128 against 0.3 ms
-  // for the upload and both kernels; a second launch and wait cost 8 us, which
-  // 8192 values take here); the loop then names the value.
+  // for the upload and both kernels; a second launch and wait cost 8 to 12 us);
+  // the loop then names the value.
   const bool on_device = h->ncell >= kDeviceCheck;
   int rc = on_device ? 0 : check();
   if (rc) return rc;
@@ -1187,17 +1187,25 @@ namespace {
 // Blocks up to which one state's objective is reduced by the objective kernel
 // itself (its last block adds the blocks' sums, which queue for one counter)
 // instead of through the warp partials, their zeroing and a summing kernel:
-// one step of a 64x48 channel with its objective took 40 us that way, 26 so.
+// one step of a 64x48 channel with its objective takes 26 us so and 40 that way.
 constexpr unsigned kDirectBlocks = 2048;
+// Steps up to which a batch's objectives are reduced so, in every step, and a
+// handle's reach the host in its own page instead of by a copy.
+constexpr int kFewSteps = 4;
 
 // lbm_forward with the objective of every step: each step adds into a row of
 // warp partials of its own, and one kernel sums the rows of up to 64 steps.
 // (A reduction to one value in every step, through a counter that all blocks
 // queue for, cost the 250x121x115 FP16 duct 128 us a step against 85 without.)
 int forward_per_step(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) {
-  int rc = ensure_jcap(h, (size_t)nsteps);
+  // few values go into the handle's page, which saves the copy (one step of a 64x48
+  // FP32 channel 40 us with it)
+  const bool few = nsteps <= kFewSteps;
+  int rc = few ? 0 : ensure_jcap(h, (size_t)nsteps);
   if (!rc) rc = ensure_step_rows(h);
   if (rc) return rc;
+  if (few) CUDA_OR_FAIL(h, h->jmap.take());
+  double* const out = few ? h->jmap.dev + kFewSteps : h->jdev;
   const size_t cap = h->partial_cap;
   int row = 0, done = 0;   // rows in use, values summed
   // the next objective's row; before the first one, after the rows are summed
@@ -1212,7 +1220,7 @@ int forward_per_step(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) 
   };
   auto sum_rows = [&](bool last) -> int {
     if (row < h->step_rows && !last) return 0;
-    k_sum_partials<<<row, 1024, 0, h->stream>>>(h->step_partial, (long long)cap, h->jdev + done);
+    k_sum_partials<<<row, 1024, 0, h->stream>>>(h->step_partial, (long long)cap, out + done);
     h->launches++;
     CUDA_OR_FAIL(h, cudaGetLastError());
     done += row;
@@ -1223,17 +1231,20 @@ int forward_per_step(lbm_handle* h, int nsteps, double* J_steps, double* J_sum) 
   for (int k = 0; k < nsteps && !rc; ++k) {
     // step k evaluates the state that step k-1 made
     if (k > 0 && (rc = next_row())) break;
-    if ((rc = forward_step(h, k > 0 ? h->jdev : nullptr))) break;
+    if ((rc = forward_step(h, k > 0 ? out : nullptr))) break;
     if (k > 0) rc = sum_rows(false);
   }
   if (!rc) rc = next_row();
-  if (!rc) rc = objective_only(h, h->jdev);
+  if (!rc) rc = objective_only(h, out);
   if (!rc) rc = sum_rows(true);
   h->accumulate = false;
   h->step_row = nullptr;
   if (rc || (rc = sync(h))) return rc;
   std::vector<double> js((size_t)nsteps);
-  CUDA_OR_FAIL(h, cudaMemcpy(js.data(), h->jdev, js.size() * sizeof(double), cudaMemcpyDeviceToHost));
+  if (few)
+    memcpy(js.data(), h->jmap.host + kFewSteps, js.size() * sizeof(double));
+  else
+    CUDA_OR_FAIL(h, cudaMemcpy(js.data(), h->jdev, js.size() * sizeof(double), cudaMemcpyDeviceToHost));
   double acc = 0.;
   for (int k = 0; k < nsteps; ++k) acc += js[k];
   if (!std::isfinite(acc)) return fail(h, LBM_ERR_NONFINITE, "objective is not finite");
@@ -2346,20 +2357,27 @@ int lbm_batch_forward(lbm_batch* b, int nsteps, double* J) {
   for (int i = 0; i < b->n; ++i) {
     if (!b->h[i]->have_design || !b->h[i]->have_state)
       return bfail(b, LBM_ERR_STATE, "lattice %d has no design or state", i);
-    if (ensure_jcap(b->h[i], 1)) return bfail(b, LBM_ERR_MEM, "%s", b->h[i]->err.c_str());
+    if (ensure_jcap(b->h[i], kFewSteps)) return bfail(b, LBM_ERR_MEM, "%s", b->h[i]->err.c_str());
   }
-  // objectives summed in the warp partials, as a gradient's forward sweep does
+  // objectives summed in the warp partials, as a gradient's forward sweep does; those
+  // of a few steps are reduced by the kernels that evaluate them (one step of four
+  // 64x48 channels 61 us, 87 with each lattice's partials zeroed and summed)
   int rc = 0;
+  bool direct = nsteps <= kFewSteps;
   double* res[LBM_MAX_BATCH];
   for (int i = 0; i < b->n; ++i) {
     res[i] = b->h[i]->jdev;
+    direct = direct && b->h[i]->geo.nblocks <= kDirectBlocks;
   }
-  for (int i = 0; i < b->n && !rc; ++i)
+  for (int i = 0; i < b->n && !rc && !direct; ++i)
     if (b->h[i]->cfg.objective != LBM_OBJ_NONE && (rc = begin_accumulate(b->h[i], b->stream)))
       bfail(b, rc, "%s", b->h[i]->err.c_str());
-  for (int s = 0; s < nsteps && !rc; ++s) rc = batch_forward(b, s >= 1 ? res : nullptr);
+  for (int s = 0; s < nsteps && !rc; ++s) {
+    rc = batch_forward(b, s >= 1 ? res : nullptr);
+    for (int i = 0; i < b->n && direct && s >= 1; ++i) ++res[i];
+  }
   if (!rc) rc = batch_objective(b, kCurState, res);
-  for (int i = 0; i < b->n && !rc; ++i)
+  for (int i = 0; i < b->n && !rc && !direct; ++i)
     if (b->h[i]->cfg.objective != LBM_OBJ_NONE &&
         (rc = end_accumulate(b->h[i], b->h[i]->jdev, b->stream)))
       bfail(b, rc, "%s", b->h[i]->err.c_str());
@@ -2368,8 +2386,11 @@ int lbm_batch_forward(lbm_batch* b, int nsteps, double* J) {
   BCUDA(b, cudaStreamSynchronize(b->stream));
   for (int i = 0; J && i < b->n; ++i) {
     J[i] = 0.;
-    if (b->h[i]->cfg.objective != LBM_OBJ_NONE)
-      BCUDA(b, cudaMemcpy(&J[i], b->h[i]->jdev, sizeof(double), cudaMemcpyDeviceToHost));
+    if (b->h[i]->cfg.objective == LBM_OBJ_NONE) continue;
+    double js[kFewSteps];
+    const int values = direct ? nsteps : 1;
+    BCUDA(b, cudaMemcpy(js, b->h[i]->jdev, values * sizeof(double), cudaMemcpyDeviceToHost));
+    for (int k = 0; k < values; ++k) J[i] += js[k];
   }
   return LBM_OK;
 }
